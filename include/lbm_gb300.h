@@ -466,6 +466,69 @@ int lbm_one_time_step_periodic(const void* f, void* fnew, const lbm_lattice* lat
 int lbm_one_time_step_walls(const void* f, void* fnew, const lbm_lattice* lat, const double* prm,
                             const double* table, const int32_t* sym, void* stream);
 
+/* Several steps in one launch, for 2D lattices of shifted (FP32-computed)
+ * storage whose stencil reaches one node.  Each block keeps a region of the
+ * grid in shared memory, advances it and writes the part that stays valid, so
+ * a launch reads and writes the populations once for all its steps; the
+ * populations are those of single launches bit for bit.  mode:
+ *   LBM_TILE_PERIODIC  periodic along every axis (lbm_one_time_step_periodic)
+ *   LBM_TILE_WALLS     bounce-back box walls (lbm_one_time_step_walls, with
+ *                      its table and sym)
+ *   LBM_TILE_LINKS     boundary links (lbm_boundary_batch, then
+ *                      lbm_one_time_step), given per tile: see lbm_tile_link
+ *
+ * lbm_scheme_multi_step_plan chooses the regions of a lattice: shape -1 takes
+ * the rule on its size (margin then ignored), else a region shape by number
+ * with `margin`, the most steps of a launch.  plan->shape is -1 where single
+ * steps are to be used (another dimension, reach, storage or size).
+ *
+ * lbm_scheme_multi_step advances `steps` steps (even) from f in an even
+ * number of launches between f and fnew, so that the result lies in f.
+ * No reference counterpart. */
+enum { LBM_TILE_PERIODIC = 0, LBM_TILE_WALLS = 1, LBM_TILE_LINKS = 2 };
+
+typedef struct lbm_tile_plan {
+  int32_t shape;     /* region shape, or -1 */
+  int32_t margin;    /* most steps of one launch */
+  int32_t out[2];    /* rows and columns a block writes */
+  int32_t tiles[2];  /* blocks along each axis */
+  int32_t pitch;     /* elements between rows of the region in shared memory */
+  int32_t plane;     /* elements between populations there */
+} lbm_tile_plan;
+
+/* One boundary link of one tile: element offsets in the region of the slot it
+ * stores and of its loads, in the plain layout [0] (f_k(x) at k * plane +
+ * (row + 1) * pitch + column + 1) and in the swapped one [1] (f_k(x) in the
+ * slot of k', opposite to k, at x + v_k); rhs and dist in the FP32 form of
+ * LBM_BC_FLOAT_FORM. */
+#define LBM_TILE_LINK_ANTI 1
+#define LBM_TILE_LINK_BOUZIDI 2
+#define LBM_TILE_LINK_COPY 4
+typedef struct lbm_tile_link {
+  uint16_t store[2];
+  uint16_t load0[2];
+  uint16_t load1[2];
+  uint32_t flags;
+  float rhs;
+  float dist;
+} lbm_tile_link;
+
+/* Boundary of a multi-step launch: table and sym (walls); first (tiles + 1
+ * link indices), links (both device) and periodic axes (links). */
+typedef struct lbm_tile_boundary {
+  const double* table;
+  const int32_t* sym;
+  const int32_t* first;
+  const lbm_tile_link* links;
+  int32_t wrap[2];
+} lbm_tile_boundary;
+
+int lbm_scheme_multi_step_plan(const lbm_lattice* lat, int32_t mode, int32_t shape, int32_t margin,
+                               lbm_tile_plan* plan);
+int lbm_scheme_multi_step(void* f, void* fnew, const lbm_lattice* lat, const double* prm,
+                          const lbm_tile_plan* plan, int32_t steps, int32_t mode,
+                          const lbm_tile_boundary* boundary, void* stream);
+
 /* Step kernel choice of this module: 1 runs periodic steps of 16-bit
  * storage in the staged kernel where the rows allow it (bulk copies of each
  * pulled row into shared memory on the TMA unit, ahead of the compute), 0

@@ -536,3 +536,129 @@ def box_wall_table(methods, shape_in, halo, velocities, constants):
     if slots.size != expected or np.unique(slots).size != slots.size:
         return None
     return table
+
+
+TILE_LINK = np.dtype([("store", np.uint16, 2), ("load0", np.uint16, 2), ("load1", np.uint16, 2),
+                      ("flags", np.uint32), ("rhs", np.float32), ("dist", np.float32)])
+_TILE_FLAGS = {"bounce_back": 0, "neumann": 0, "anti_bounce_back": 1, "bouzidi_bounce_back": 2,
+               "bouzidi_anti_bounce_back": 3}
+
+
+def tile_links(entries, ghost, shape_in, halo, wrap, velocities, opposite, plan):
+    """The links of a batched boundary launch, by the tiles of a multi-step
+    launch (lbm_scheme_multi_step): (first, links) with the lbm_tile_link
+    records of tile t in links[first[t]:first[t + 1]], or None where the links
+    do not fit the tiles.
+
+    ``entries``: dicts with kind, iload (lists of (k, i0, i1) slots), istore,
+    rhs and dist (FP32 form) of a batch in which no link reads a slot that
+    another stores; ``ghost``: (istore, iload) of the observed ghost copies
+    joined to it, or None; ``wrap``: periodic axes; ``opposite``: the
+    population of the opposite velocity; ``plan``: lbm_tile_plan.
+
+    A link is known by the node x that pulls its slot: x = slot + v_k.  Every
+    tile that advances x carries the link, at the place of x (and of its
+    periodic images) in the tile's region.  A node e rows or columns outside
+    the tile's output is needed at the steps that leave at least e steps to
+    go, so a link's loads may lie at most one further out than x.  A periodic
+    axis is wrapped by the region itself, so copies of periodic images are
+    dropped; any other ghost copy, or a load outside the grid, returns None.
+    """
+    n = np.asarray(shape_in, dtype=np.int64)
+    h = np.asarray(halo, dtype=np.int64)
+    wrap = np.asarray(wrap, dtype=bool)
+    vel = np.asarray(velocities, dtype=np.int64)
+    opposite = np.asarray(opposite, dtype=np.int64)
+    if ghost is not None:
+        st, il = (np.asarray(a, dtype=np.int64) for a in ghost)
+        c = st[:, 1:] - h
+        outside = (c < 0) | (c >= n)
+        image = np.where(wrap & outside, c % n, c)
+        if (outside & ~wrap).any() or not np.array_equal(image, il[:, 1:] - h) or not np.array_equal(st[:, 0], il[:, 0]):
+            return None
+    out, tiles = np.array(plan.out[:], dtype=np.int64), np.array(plan.tiles[:], dtype=np.int64)
+    margin = int(plan.margin)
+    region = out + 2 * margin
+    keys, rows = [], []
+    for e in entries:
+        st = np.asarray(e["istore"], dtype=np.int64)
+        x = st[:, 1:] - h + vel[st[:, 0]]
+        keep = ((x >= 0) & (x < n)).all(axis=1)     # slots that a node of the grid pulls
+        if not keep.any():
+            continue
+        st, x = st[keep], x[keep]
+        loads = []
+        for il in e["iload"]:
+            il = np.asarray(il, dtype=np.int64)[keep]
+            y = il[:, 1:] - h
+            d = y - x
+            d = np.where(wrap, (d + n // 2) % n - n // 2, d)   # the image nearest to x
+            y = x + d
+            if (np.abs(d) > 3).any() or (((y < 0) | (y >= n)) & ~wrap).any():
+                return None
+            loads.append((il[:, 0], d))
+        # every region place of x along each axis: link, tile index and place.
+        # Tile t holds the coordinates t out - margin + [0, region)
+        places = []
+        for a in range(2):
+            images = [0]
+            if wrap[a]:
+                reach = int(region[a] // n[a]) + 1
+                images = range(-reach, reach + 1)
+            parts = []
+            for im in images:
+                c = x[:, a] + im * n[a] + margin
+                last = c // out[a]
+                for back in range(int(-(-region[a] // out[a]))):
+                    t = last - back
+                    r = c - t * out[a]
+                    i = np.flatnonzero((t >= 0) & (t < tiles[a]) & (r < region[a]))
+                    if i.size:
+                        parts.append((i, t[i], r[i]))
+            if not parts:
+                parts = [(np.zeros(0, np.int64),) * 3]
+            i_all = np.concatenate([p[0] for p in parts])
+            order = np.argsort(i_all, kind="stable")
+            places.append([i_all[order]] + [np.concatenate([p[j] for p in parts])[order] for j in (1, 2)])
+        # all pairs of places of one link along the two axes
+        (i0, t0, r0), (i1, t1, r1) = places
+        c1 = np.bincount(i1, minlength=len(st))
+        s1 = np.concatenate([[0], np.cumsum(c1)])
+        reps = c1[i0]
+        a0 = np.repeat(np.arange(len(i0)), reps)
+        a1 = np.arange(reps.sum()) - np.repeat(np.cumsum(reps) - reps, reps) + np.repeat(s1[i0], reps)
+        link, row, col = i0[a0], r0[a0], r1[a1]
+        tile = t0[a0] * tiles[1] + t1[a1]
+
+        def away(r, c):
+            return np.maximum(np.maximum(margin - r, r - (margin + out[0] - 1)),
+                              np.maximum(margin - c, c - (margin + out[1] - 1))).clip(0)
+
+        need = away(row, col) < margin
+        link, row, col, tile = link[need], row[need], col[need], tile[need]
+        ahead = away(row, col) + 1
+        rec = np.zeros(len(link), dtype=TILE_LINK)
+
+        def place(field, k, r, c):
+            o, v = opposite[k], vel[k]
+            rec[field][:, 0] = k * plan.plane + (r + 1) * plan.pitch + c + 1
+            rec[field][:, 1] = o * plan.plane + (r + 1 + v[:, 0]) * plan.pitch + c + 1 + v[:, 1]
+
+        k = st[link, 0]
+        place("store", k, row - vel[k, 0], col - vel[k, 1])
+        for field, (kl, d) in zip(("load0", "load1"), loads):
+            r, c = row + d[link, 0], col + d[link, 1]
+            if (away(r, c) > ahead).any():
+                return None
+            place(field, kl[link], r, c)
+        rec["flags"] = _TILE_FLAGS[e["kind"]]
+        rec["rhs"] = np.asarray(e["rhs"], dtype=np.float32)[keep][link]
+        if e.get("dist") is not None:
+            rec["dist"] = np.asarray(e["dist"], dtype=np.float32)[keep][link]
+        keys.append(tile)
+        rows.append(rec)
+    tile = np.concatenate(keys) if keys else np.zeros(0, np.int64)
+    rec = np.concatenate(rows) if rows else np.zeros(0, TILE_LINK)
+    order = np.argsort(tile, kind="stable")
+    first = np.concatenate([[0], np.cumsum(np.bincount(tile, minlength=int(tiles.prod())))]).astype(np.int32)
+    return first, np.ascontiguousarray(rec[order])

@@ -233,6 +233,23 @@ def _cheaper(a, b):
     return b if sp.count_ops(b) < sp.count_ops(a) else a
 
 
+def opposite_populations(v):
+    """k' of every population k with v[k'] = -v[k], one to one (the i-th
+    population of a velocity with the i-th of the opposite one), or None."""
+    rows = [tuple(int(c) for c in row) for row in v]
+    where = {}
+    for k, row in enumerate(rows):
+        where.setdefault(row, []).append(k)
+    out = [0] * len(rows)
+    for row, ks in where.items():
+        back = where.get(tuple(-c for c in row), [])
+        if len(back) != len(ks):
+            return None
+        for a, b in zip(ks, back):
+            out[a] = b
+    return out
+
+
 class SchemeSource:
     """Generated device code for one scheme and one storage form.
 
@@ -592,6 +609,11 @@ class SchemeSource:
         out.append(f"#define LBM_VMAX {max(vmax, 1)}")
         out.append("#define LBM_FOR_EACH_V(X) " + " ".join(
             f"X({k}, {int(v[k, 0])}, {int(v[k, 1])}, {int(v[k, 2])})" for k in range(nv)))
+        opposite = opposite_populations(v)
+        if opposite is not None:
+            # every population with one of the opposite velocity: X(k, vx, vy, vz, k')
+            out.append("#define LBM_FOR_EACH_AA(X) " + " ".join(
+                f"X({k}, {int(v[k, 0])}, {int(v[k, 1])}, {int(v[k, 2])}, {opposite[k]})" for k in range(nv)))
         out.append("__device__ __constant__ double lbm_dev_shift[LBM_Q] = {" +
                    ", ".join(repr(float(x)) for x in self.shift) + "};")
         out.append("__device__ __constant__ double lbm_dev_mref[LBM_Q] = {" +
@@ -704,7 +726,8 @@ class SchemeSource:
                  and compute == "float32")
         return (f"#define LBM_STORAGE {ctypes_[storage]}\n"
                 f"#define LBM_COMPUTE {ctypes_[compute]}\n"
-                + ("#define LBM_PAIRS 1\n" if pairs else "") +
+                + ("#define LBM_PAIRS 1\n" if pairs else "")
+                + ("#define LBM_FLOAT_COMPUTE 1\n" if compute == "float32" else "") +
                 "#include \"lbm_common.cuh\"\n"
                 "using lbm::lbm_fma;\n"
                 "template <typename R> __device__ __forceinline__ R lbm_sqrt(R x) { return sqrt(x); }\n"

@@ -1277,6 +1277,8 @@ __global__ void __launch_bounds__(LBM_BLOCK) k_source_term(double* __restrict__ 
   for (int k = 0; k < LBM_NCONS; ++k) m[om + (long long)k * a.gm.vstride] = mm[k];
 }
 
+#include "tile_steps.cuh"
+
 // ------------------------------------------------------------------ host
 // need_halo: the stencil reach in ghost layers, for the kernels that pull
 // neighbours; the pointwise transforms (f2m, m2f) take any halo, including
@@ -1785,3 +1787,224 @@ int lbm_relaxation(double* m, const lbm_lattice* mlat, const double* prm, void* 
 }
 
 }  // extern "C"
+
+#if LBM_HAS_TILE_STEPS
+namespace lbm_scheme {
+
+// Region shapes of the multi-step launch.  64 x 32 with two blocks an SM is
+// the fastest where there are several regions per SM (1024^2 D2Q9 FP32: 6.9 us
+// a step against 13.3 one step at a time); 64 x 48, one block an SM, where one
+// region per SM covers the grid (512^2: 2.3 against 5.1 us); 32 x 32 below
+// (256^2: 1.05 against 3.9 us).  All of it is issue-bound: 32 x 16, 64 x 64,
+// 1024 threads at 32 registers and two rows per thread in packed FP32x2
+// arithmetic (as many FMA-pipe cycles, constants in register pairs) were
+// within 5 % of these or slower.
+using Tile0 = TileShape<64, 32, 512, 2>;
+using Tile1 = TileShape<64, 48, 768, 1>;
+using Tile2 = TileShape<32, 32, 512, 3>;
+constexpr int kTileShapes = 3;
+constexpr size_t kTileMaxBytes = 220 * 1024;
+
+template <class F>
+inline int with_tile_shape(int shape, F&& fn) {
+  switch (shape) {
+    case 0: return fn(Tile0());
+    case 1: return fn(Tile1());
+    case 2: return fn(Tile2());
+    default: return LBM_ERR_ARG;
+  }
+}
+
+// shared memory above 48 KB is granted per kernel and device, once (static:
+// a function-local static with external linkage is one object for all the
+// modules of a process)
+template <class Shape, int kMode>
+static int tile_grant(const char* who) {
+  static bool done[64];
+  int dev = 0;
+  int rc = lbm::cuda_check(cudaGetDevice(&dev), who);
+  if (rc || (dev >= 0 && dev < 64 && done[dev])) return rc;
+  rc = lbm::cuda_check(cudaFuncSetAttribute(k_steps_tile<Shape, kMode>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                            (int)Shape::kBytes),
+                       who);
+  if (!rc && dev >= 0 && dev < 64) done[dev] = true;
+  return rc;
+}
+
+// The region shape and margin of a lattice, by the time they are expected to
+// take (D2Q9 FP32 launches of every shape and margin at 96^2 to 1536^2 keep to
+// it within about 10 %): kLaunchUs for a launch with its first loads, then on
+// the busiest SM the rows its regions still need at every step, kRate
+// lane-nodes a microsecond.  Where several blocks share an SM one's loads run
+// beside another's steps, and 0.6 (16 bits: 0.75) of the steps' time and 0.75 of the traffic's
+// at 5 TB/s remain.  Single steps stay (shape -1) where they are expected to be
+// no slower; for 16-bit storage, whose two-node step moves half the bytes,
+// from 1.5 10^6 nodes on (1536^2 FP16: 15.4 us a step against 15.6).
+inline void tile_rule(const lbm_lattice& lat, int& shape, int& margin) {
+  constexpr bool kHalf = sizeof(S) == 2;
+  constexpr double kLaunchUs = 2.6, kRate = kHalf ? 1350.0 : 1600.0;
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1) {
+    (void)cudaGetLastError();
+    sms = 152;
+  }
+  const double nodes = (double)lat.n[0] * lat.n[1];
+  double best = kHalf ? (nodes < 1.5e6 ? 1.9 + 6.0e-6 * nodes : 0.0) : kLaunchUs + 10e-6 * nodes;
+  shape = -1;
+  for (int s = 0; s < kTileShapes; ++s)
+    with_tile_shape(s, [&](auto tag) {
+      using Shape = decltype(tag);
+      if (Shape::kBytes > kTileMaxBytes) return 0;
+      for (int m = 2; m <= 10; ++m) {
+        const int o0 = Shape::kH - 2 * m, o1 = Shape::kW - 2 * m;
+        if (o0 < 8 || o1 < 8) break;
+        const double tiles = (double)((lat.n[0] + o0 - 1) / o0) * ((lat.n[1] + o1 - 1) / o1);
+        const double waves = (double)(((long long)tiles + sms - 1) / sms);
+        const double rows = (double)m * Shape::kH - m * (m + 1.0);  // sum of kH - 2 s over the steps
+        const double bytes = (tiles * Shape::kW * Shape::kH + nodes) * LBM_Q * sizeof(S);
+        const double work = waves * rows * Shape::kW / kRate;
+        const double us = (kLaunchUs + (waves == 1.0         ? work
+                                        : Shape::kBlocks > 1 ? (kHalf ? 0.75 : 0.6) * work + 0.75 * bytes / 5e6
+                                                             : work + 1.5 * waves)) / m;
+        if (us < best) {
+          best = us;
+          shape = s;
+          margin = m;
+        }
+      }
+      return 0;
+    });
+}
+
+}  // namespace lbm_scheme
+#endif
+
+extern "C" int lbm_scheme_multi_step_plan(const lbm_lattice* lat, int32_t mode, int32_t shape, int32_t margin,
+                                   lbm_tile_plan* plan) {
+  using namespace lbm_scheme;
+  const char* who = "lbm_scheme_multi_step_plan";
+  int rc = check_pop_lattice(lat, who);
+  if (rc) return rc;
+  if (!plan) return lbm::fail(LBM_ERR_ARG, "%s: NULL plan", who);
+  if (mode < 0 || mode > 2) return lbm::fail(LBM_ERR_ARG, "%s: mode %d", who, mode);
+  plan->shape = -1;
+  plan->margin = 0;
+  plan->out[0] = plan->out[1] = plan->tiles[0] = plan->tiles[1] = plan->pitch = plan->plane = 0;
+#if LBM_HAS_TILE_STEPS
+  if (lat->elements >= (1LL << 31)) return LBM_OK;  // the kernel indexes with 32 bits
+  if (shape >= kTileShapes) return lbm::fail(LBM_ERR_ARG, "%s: shape %d", who, shape);
+  if (shape < 0) {
+    tile_rule(*lat, shape, margin);
+    if (shape < 0) return LBM_OK;
+  }
+  return with_tile_shape(shape, [&](auto tag) {
+    using Shape = decltype(tag);
+    if (Shape::kBytes > kTileMaxBytes) return (int)LBM_OK;
+    if (margin < 1 || 2 * margin >= Shape::kH || 2 * margin >= Shape::kW)
+      return lbm::fail(LBM_ERR_ARG, "%s: margin %d", who, margin);
+    const int room[2] = {Shape::kH - 2 * margin, Shape::kW - 2 * margin};
+    for (int d = 0; d < 2; ++d) {
+      plan->tiles[d] = (lat->n[d] + room[d] - 1) / room[d];
+      plan->out[d] = (lat->n[d] + plan->tiles[d] - 1) / plan->tiles[d];  // tiles of one size
+    }
+    if (plan->tiles[0] > 65535) return (int)LBM_OK;
+    plan->shape = shape;
+    plan->margin = margin;
+    plan->pitch = Shape::kPitch;
+    plan->plane = Shape::kPlane;
+    return (int)LBM_OK;
+  });
+#else
+  (void)shape;
+  (void)margin;
+  return LBM_OK;
+#endif
+}
+
+extern "C" int lbm_scheme_multi_step(void* f, void* fnew, const lbm_lattice* lat, const double* prm,
+                                     const lbm_tile_plan* plan, int32_t steps, int32_t mode,
+                                     const lbm_tile_boundary* boundary, void* stream) {
+  using namespace lbm_scheme;
+  const char* who = "lbm_scheme_multi_step";
+  int rc = check_pop_lattice(lat, who);
+  if (rc) return rc;
+  if (!f || !fnew || f == fnew) return lbm::fail(LBM_ERR_ARG, "%s: bad population buffers", who);
+  if (!plan) return lbm::fail(LBM_ERR_ARG, "%s: NULL plan", who);
+  if (LBM_NPRM > 0 && !prm) return lbm::fail(LBM_ERR_ARG, "%s: %d parameters expected", who, LBM_NPRM);
+  if (mode < 0 || mode > 2) return lbm::fail(LBM_ERR_ARG, "%s: mode %d", who, mode);
+#if LBM_HAS_TILE_STEPS
+  if (lat->elements >= (1LL << 31)) return lbm::fail(LBM_ERR_UNSUPPORTED, "%s: lattice too large", who);
+  if (plan->shape < 0 || plan->shape >= kTileShapes || plan->margin < 1 || steps < 2 || steps % 2)
+    return lbm::fail(LBM_ERR_ARG, "%s: shape %d, margin %d, %d steps", who, plan->shape, plan->margin, steps);
+  const bool walls = mode == LBM_TILE_WALLS, linked = mode == LBM_TILE_LINKS;
+  if ((walls && (!boundary || !boundary->table || !boundary->sym)) ||
+      (linked && (!boundary || !boundary->first || !boundary->links)))
+    return lbm::fail(LBM_ERR_ARG, "%s: NULL boundary", who);
+  StepArgs sa = make_step_args(*lat, prm);
+  TileArgs a;
+  for (int d = 0; d < 2; ++d) {
+    a.n[d] = lat->n[d];
+    a.out[d] = plan->out[d];
+    a.wrap[d] = linked ? boundary->wrap[d] : mode == LBM_TILE_PERIODIC;
+    if (plan->out[d] < 1 || plan->tiles[d] < 1 || (long long)plan->out[d] * plan->tiles[d] < lat->n[d])
+      return lbm::fail(LBM_ERR_ARG, "%s: tiles do not cover axis %d", who, d);
+  }
+  a.stride0 = (int)lat->stride[0];
+  a.vstride = (int)lat->vstride;
+  a.base = (int)(lat->origin + lat->halo[0] * lat->stride[0] + lat->halo[1]);
+  a.margin = plan->margin;
+  a.first = linked ? boundary->first : nullptr;
+  a.links = linked ? boundary->links : nullptr;
+  for (int i = 0; i < kPrm; ++i) a.prm[i] = sa.prm[i];
+  WallArgs w;
+  if (walls) {
+    for (int d = 0; d < 2; ++d)
+      if (lat->halo[d] != 1) return lbm::fail(LBM_ERR_ARG, "%s: halo[%d]=%d, one ghost layer expected", who, d, lat->halo[d]);
+    // the swapped layout pairs the populations as the walls do
+#define LBM_TILE_SYM(k, vx, vy, vz, ko) \
+  if (boundary->sym[k] != (ko)) return lbm::fail(LBM_ERR_UNSUPPORTED, "%s: sym[%d]=%d", who, (k), boundary->sym[k]);
+    LBM_FOR_EACH_AA(LBM_TILE_SYM)
+#undef LBM_TILE_SYM
+    for (int k = 0; k < LBM_Q; ++k) {
+      w.sym[k] = boundary->sym[k];
+      for (int j = 0; j < 27; ++j) w.c[k][j] = (R)boundary->table[k * 27 + j];
+    }
+  }
+  return with_tile_shape(plan->shape, [&](auto tag) {
+    using Shape = decltype(tag);
+    if (Shape::kBytes > kTileMaxBytes || plan->out[0] + 2 * plan->margin > Shape::kH ||
+        plan->out[1] + 2 * plan->margin > Shape::kW || plan->pitch != Shape::kPitch || plan->plane != Shape::kPlane)
+      return lbm::fail(LBM_ERR_ARG, "%s: tile %d x %d with margin %d", who, plan->out[0], plan->out[1], plan->margin);
+    int r = walls ? tile_grant<Shape, kTileWalls>(who)
+                  : linked ? tile_grant<Shape, kTileLinks>(who) : tile_grant<Shape, kTilePeriodic>(who);
+    if (r) return r;
+    const dim3 grid((unsigned)plan->tiles[1], (unsigned)plan->tiles[0]);
+    cudaStream_t st = (cudaStream_t)stream;
+    // an even number of launches, their steps as equal as they go
+    const int launches = 2 * ((steps + 2 * plan->margin - 1) / (2 * plan->margin));
+    S* from = (S*)f;
+    S* to = (S*)fnew;
+    for (int i = 0; i < launches; ++i) {
+      a.steps = (int)((long long)steps * (i + 1) / launches - (long long)steps * i / launches);
+      if (walls)
+        k_steps_tile<Shape, kTileWalls><<<grid, Shape::kThreads, Shape::kBytes, st>>>(from, to, a, w);
+      else if (linked)
+        k_steps_tile<Shape, kTileLinks><<<grid, Shape::kThreads, Shape::kBytes, st>>>(from, to, a, w);
+      else
+        k_steps_tile<Shape, kTilePeriodic><<<grid, Shape::kThreads, Shape::kBytes, st>>>(from, to, a, w);
+      r = lbm::launch_check(who);
+      if (r) return r;
+      S* t = from;
+      from = to;
+      to = t;
+    }
+    return (int)LBM_OK;
+  });
+#else
+  (void)steps;
+  (void)boundary;
+  (void)stream;
+  return lbm::fail(LBM_ERR_UNSUPPORTED, "%s: not available for this scheme", who);
+#endif
+}

@@ -1,0 +1,264 @@
+// Several time steps of a 2D lattice in one launch (included by
+// scheme_kernels.cuh inside lbm_scheme, after the wall fold).
+//
+// One step at a time a 2D grid is bound by what surrounds the arithmetic: a
+// 256^2 step is 2.4 MB in L2 and about 0.3 us of FP32 issue, and took 3.9 us,
+// launch and memory latency.  Here a block takes a region of the grid into
+// shared memory, advances it T steps there and writes the part that T steps
+// leave valid: T steps cost one launch, one read (of the region, halo
+// included) and one write of the populations.
+//
+// The region is kept once, not twice.  A node reads Q slots and writes its
+// new populations into the same Q slots, so no other thread touches them
+// during the step, and one barrier separates two steps:
+//   plain layout    f_k(x) lies in slot (k, x);  a node pulls (k, x - v_k)
+//   swapped layout  f_k(x) lies in slot (k', x + v_k), k' opposite to k;
+//                   a node finds f_k(x - v_k) in its own slot (k', x)
+// A step from the plain layout writes the swapped one and the reverse
+// (Bailey et al. 2009, "Accelerating lattice Boltzmann fluid flow simulations
+// using graphics processors", alternate the same two access patterns).
+//
+// A thread updates two rows of one column at a time (packed FP32x2 algebra):
+// its shared-memory accesses run along the row, one word per lane, without
+// bank conflicts or alignment rules, at any width of the grid.  Values are
+// kept in the storage type, so each step rounds as a step through HBM does,
+// and the arithmetic is the generated collide of the one-step kernels: the
+// populations after T steps are those of T single launches bit for bit.
+
+#if LBM_DIM == 2 && LBM_VMAX == 1 && defined(LBM_FOR_EACH_AA) && defined(LBM_FLOAT_COMPUTE) && LBM_Q <= 16
+#define LBM_HAS_TILE_STEPS 1
+
+constexpr int kTilePeriodic = 0, kTileWalls = 1, kTileLinks = 2;
+
+struct TileArgs {
+  int n[2];
+  int stride0;        // elements between rows
+  int vstride;        // elements between populations
+  int base;           // element offset of interior node (0, 0) of population 0
+  int steps;          // time steps of this launch, at most margin
+  int margin;         // rows and columns of the region around the output
+  int out[2];         // output rows and columns of a tile
+  int wrap[2];        // axis is periodic (the links kernel; else by mode)
+  const int* first;   // links kernel: first link of every tile, and the total
+  const lbm_tile_link* links;
+  R prm[kPrm];
+};
+
+// one value of shared memory, in FP32
+template <typename T> struct SharedValue;
+template <> struct SharedValue<float> {
+  __device__ __forceinline__ static float get(const float* p) { return *p; }
+};
+template <> struct SharedValue<__half> {
+  __device__ __forceinline__ static float get(const __half* p) { return __half2float(*p); }
+};
+template <> struct SharedValue<__nv_bfloat16> {
+  __device__ __forceinline__ static float get(const __nv_bfloat16* p) { return __bfloat162float(*p); }
+};
+
+// region shape: kW columns (a multiple of 32) x kH rows, kThreads threads;
+// a frame of one cell around it takes what border nodes read and
+// write beyond it (values that no valid node uses)
+template <int kW_, int kH_, int kThreads_, int kBlocks_>
+struct TileShape {
+  static constexpr int kBlocks = kBlocks_;  // blocks per SM the registers have to leave room for
+  static constexpr int kW = kW_, kH = kH_, kThreads = kThreads_;
+  static constexpr int kPitch = kW + 2;
+  static constexpr int kPlane = (kH + 2) * kPitch;
+  static constexpr size_t kBytes = (size_t)LBM_Q * kPlane * sizeof(S);
+  static constexpr int kWarpRows = kThreads / kW;  // rows advanced side by side
+  static_assert(kW % 32 == 0 && kThreads % kW == 0 && kH % (kThreads / kW) == 0, "whole warps and rows");
+};
+
+// grid coordinate c of an axis of n nodes, wrapped into [0, n)
+__device__ __forceinline__ int tile_wrap(int c, int n) {
+  if (c >= 0 && c < n) return c;
+  c %= n;
+  return c < 0 ? c + n : c;
+}
+
+// step s (1-based) of the region in shared memory
+template <class Shape, int kMode, bool kSwapped, bool kLast>
+__device__ __forceinline__ void tile_step(S* __restrict__ sm, S* __restrict__ fnew, const TileArgs& a,
+                                          const R (&prm)[kPrm], const WallArgs* w, int i0s, int i1s,
+                                          int s) {
+  const int col = threadIdx.x % Shape::kW;
+  const int used = a.out[0] + 2 * a.margin;  // rows of the region that this tile needs
+  const int g1 = i1s + col;
+  const bool in1 = kMode == kTilePeriodic || (g1 >= 0 && g1 < a.n[1]) || (kMode == kTileLinks && a.wrap[1]);
+  // columns the output or a later step needs
+  if (!in1 || col < s || col >= a.out[1] + 2 * a.margin - s) return;
+  for (int r = threadIdx.x / Shape::kW; r < Shape::kH; r += Shape::kWarpRows) {
+    const int g0 = i0s + r;
+    if (r < s || r >= used - s) continue;
+    if ((kMode == kTileWalls || (kMode == kTileLinks && !a.wrap[0])) && (g0 < 0 || g0 >= a.n[0])) continue;
+    S* p = sm + (r + 1) * Shape::kPitch + col + 1;
+    R g[LBM_Q];
+#define LBM_TILE_GET(k, vx, vy, vz, ko) \
+  g[k] = SharedValue<S>::get(kSwapped ? p + (ko) * Shape::kPlane : p + ((k) * Shape::kPlane - (vx) * Shape::kPitch - (vy)));
+    LBM_FOR_EACH_AA(LBM_TILE_GET)
+#undef LBM_TILE_GET
+    bool edge = false;
+    if (kMode == kTileWalls) {
+      const bool lo0 = g0 == 0, hi0 = g0 == a.n[0] - 1, lo1 = g1 == 0, hi1 = g1 == a.n[1] - 1;
+      edge = lo0 || hi0 || lo1 || hi1;
+      if (edge) {
+        // f_k'(x) + c in place of what would come from beyond a wall; in both
+        // layouts f_k'(x) lies in slot (k', x)
+#define LBM_TILE_WALL(k, vx, vy, vz, ko)                                                                \
+  {                                                                                                     \
+    const int sig = 9 * (wall_off(vx, lo0, hi0) + 1) + 3 * (wall_off(vy, lo1, hi1) + 1) + 1;            \
+    if (sig != 13) g[k] = through_storage(SharedValue<S>::get(p + (ko) * Shape::kPlane) + w->c[k][sig]); \
+  }
+        LBM_FOR_EACH_AA(LBM_TILE_WALL)
+#undef LBM_TILE_WALL
+      }
+    }
+    lbm_collide<R>(g, prm);
+    if (kLast) {
+      // the valid part of the region: output rows and columns (a tile may
+      // reach beyond the grid)
+      const int c0 = r - a.margin, c1 = col - a.margin;
+      if (c0 < 0 || c0 >= a.out[0] || g0 >= a.n[0] || c1 < 0 || c1 >= a.out[1] || g1 >= a.n[1]) continue;
+      S* d = fnew + (a.base + g0 * a.stride0 + g1);
+#pragma unroll
+      for (int k = 0; k < LBM_Q; ++k) Store<S>::store(d + k * a.vstride, g[k]);
+    } else if (kMode != kTileWalls || !edge) {
+#define LBM_TILE_PUT(k, vx, vy, vz, ko) \
+  Store<S>::store(kSwapped ? p + (k) * Shape::kPlane : p + ((ko) * Shape::kPlane + (vx) * Shape::kPitch + (vy)), g[k]);
+      LBM_FOR_EACH_AA(LBM_TILE_PUT)
+#undef LBM_TILE_PUT
+    } else {
+      // a population that leaves the box stays in the node's own slot (k, x)
+#define LBM_TILE_PUT_WALL(k, vx, vy, vz, ko)                                                                    \
+  {                                                                                                             \
+    const bool stay = kSwapped || g0 + (vx) < 0 || g0 + (vx) >= a.n[0] || g1 + (vy) < 0 || g1 + (vy) >= a.n[1]; \
+    Store<S>::store(p + (stay ? (k) * Shape::kPlane : (ko) * Shape::kPlane + (vx) * Shape::kPitch + (vy)), g[k]); \
+  }
+      LBM_FOR_EACH_AA(LBM_TILE_PUT_WALL)
+#undef LBM_TILE_PUT_WALL
+    }
+  }
+}
+
+// the values the boundary methods give the slots of this tile, before a step
+// reads them (kSwapped: the layout the step reads).  No link reads a slot that
+// another one stores (the host's plan), so one pass needs no order.
+template <bool kSwapped>
+__device__ __forceinline__ void tile_links(S* __restrict__ sm, const TileArgs& a, int begin, int end) {
+  for (int i = begin + (int)threadIdx.x; i < end; i += (int)blockDim.x) {
+    const lbm_tile_link l = a.links[i];
+    const float g0 = SharedValue<S>::get(sm + l.load0[kSwapped]);
+    float v;
+    if (l.flags & LBM_TILE_LINK_BOUZIDI) {
+      const float g1 = SharedValue<S>::get(sm + l.load1[kSwapped]);
+      const float t1 = __fmul_rn(__fsub_rn(1.0f, l.dist), g1);
+      const float t0 = __fmul_rn(l.dist, g0);
+      v = __fadd_rn(l.flags & LBM_TILE_LINK_ANTI ? __fsub_rn(t1, t0) : __fadd_rn(t1, t0), l.rhs);
+    } else if (l.flags & LBM_TILE_LINK_COPY) {
+      v = g0;
+    } else {
+      v = __fadd_rn(l.flags & LBM_TILE_LINK_ANTI ? -g0 : g0, l.rhs);
+    }
+    Store<S>::store(sm + l.store[kSwapped], v);
+  }
+}
+
+// the populations of the region, into the plain layout
+template <class Shape, int kMode>
+__device__ __forceinline__ void tile_load(const S* __restrict__ f, S* __restrict__ sm, const TileArgs& a, int i0s,
+                                          int i1s) {
+  const int col = threadIdx.x % Shape::kW;
+  const int used = a.out[0] + 2 * a.margin;
+  const bool wrap0 = kMode == kTilePeriodic || (kMode == kTileLinks && a.wrap[0]);
+  const bool wrap1 = kMode == kTilePeriodic || (kMode == kTileLinks && a.wrap[1]);
+  const int g1 = wrap1 ? tile_wrap(i1s + col, a.n[1]) : i1s + col;
+  if (col >= a.out[1] + 2 * a.margin || g1 < 0 || g1 >= a.n[1]) return;
+  const S* src = f + (a.base + g1);
+  // every load of the region is in flight before the first value is used
+  S v[Shape::kH / Shape::kWarpRows][LBM_Q];
+#pragma unroll
+  for (int i = 0; i < Shape::kH / Shape::kWarpRows; ++i) {
+    const int r = threadIdx.x / Shape::kW + i * Shape::kWarpRows;
+    const int g0 = wrap0 ? tile_wrap(i0s + r, a.n[0]) : i0s + r;
+    if (r >= used || g0 < 0 || g0 >= a.n[0]) continue;
+    const S* s = src + g0 * a.stride0;
+#pragma unroll
+    for (int k = 0; k < LBM_Q; ++k) v[i][k] = s[k * a.vstride];
+  }
+#pragma unroll
+  for (int i = 0; i < Shape::kH / Shape::kWarpRows; ++i) {
+    const int r = threadIdx.x / Shape::kW + i * Shape::kWarpRows;
+    if (r >= used) continue;
+    S* d = sm + (r + 1) * Shape::kPitch + col + 1;
+#pragma unroll
+    for (int k = 0; k < LBM_Q; ++k) d[k * Shape::kPlane] = v[i][k];
+  }
+}
+
+// a.steps steps of one region
+template <class Shape, int kMode>
+__device__ __forceinline__ void tile_run(const S* __restrict__ f, S* __restrict__ fnew, S* __restrict__ sm,
+                                         const TileArgs& a, const WallArgs* w, int begin, int end) {
+  const int i0s = (int)blockIdx.y * a.out[0] - a.margin;
+  const int i1s = (int)blockIdx.x * a.out[1] - a.margin;
+  R prm[kPrm];
+#pragma unroll
+  for (int p = 0; p < kPrm; ++p) prm[p] = a.prm[p];
+  tile_load<Shape, kMode>(f, sm, a, i0s, i1s);
+  int s = 1;
+#pragma unroll 1
+  while (true) {
+    __syncthreads();
+    if (kMode == kTileLinks) {
+      tile_links<false>(sm, a, begin, end);
+      __syncthreads();
+    }
+    if (s == a.steps) {
+      tile_step<Shape, kMode, false, true>(sm, fnew, a, prm, w, i0s, i1s, s);
+      return;
+    }
+    tile_step<Shape, kMode, false, false>(sm, fnew, a, prm, w, i0s, i1s, s);
+    ++s;
+    __syncthreads();
+    if (kMode == kTileLinks) {
+      tile_links<true>(sm, a, begin, end);
+      __syncthreads();
+    }
+    if (s == a.steps) {
+      tile_step<Shape, kMode, true, true>(sm, fnew, a, prm, w, i0s, i1s, s);
+      return;
+    }
+    tile_step<Shape, kMode, true, false>(sm, fnew, a, prm, w, i0s, i1s, s);
+    ++s;
+  }
+}
+
+// A region that lies inside the grid and holds no link takes the periodic
+// path in every mode: its loads wrap nowhere.
+template <class Shape, int kMode>
+__global__ void __launch_bounds__(Shape::kThreads, LBM_Q <= 9 ? Shape::kBlocks : 1)
+    k_steps_tile(const S* __restrict__ f, S* __restrict__ fnew, const __grid_constant__ TileArgs a,
+                 const __grid_constant__ WallArgs w) {
+  extern __shared__ __align__(16) unsigned char tile_smem[];
+  S* sm = reinterpret_cast<S*>(tile_smem);
+  if (kMode == kTilePeriodic) {
+    tile_run<Shape, kTilePeriodic>(f, fnew, sm, a, nullptr, 0, 0);
+    return;
+  }
+  const int r0 = (int)blockIdx.y * a.out[0] - a.margin, r1 = (int)blockIdx.x * a.out[1] - a.margin;
+  bool inside = ((kMode == kTileLinks && a.wrap[0]) || (r0 >= 0 && r0 + a.out[0] + 2 * a.margin <= a.n[0])) &&
+                ((kMode == kTileLinks && a.wrap[1]) || (r1 >= 0 && r1 + a.out[1] + 2 * a.margin <= a.n[1]));
+  int begin = 0, end = 0;
+  if (kMode == kTileLinks) {
+    const int tile = blockIdx.y * gridDim.x + blockIdx.x;
+    begin = a.first[tile];
+    end = a.first[tile + 1];
+    inside = inside && begin == end;
+  }
+  if (inside)
+    tile_run<Shape, kTilePeriodic>(f, fnew, sm, a, nullptr, 0, 0);
+  else
+    tile_run<Shape, kMode>(f, fnew, sm, a, &w, begin, end);
+}
+#endif

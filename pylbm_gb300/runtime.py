@@ -113,6 +113,34 @@ class ElementDesc(ctypes.Structure):
     ]
 
 
+class TilePlan(ctypes.Structure):
+    """lbm_tile_plan of include/lbm_gb300.h (regions of a multi-step launch)."""
+
+    _fields_ = [
+        ("shape", ctypes.c_int32),
+        ("margin", ctypes.c_int32),
+        ("out", ctypes.c_int32 * 2),
+        ("tiles", ctypes.c_int32 * 2),
+        ("pitch", ctypes.c_int32),
+        ("plane", ctypes.c_int32),
+    ]
+
+
+class TileBoundary(ctypes.Structure):
+    """lbm_tile_boundary of include/lbm_gb300.h."""
+
+    _fields_ = [
+        ("table", ctypes.c_void_p),
+        ("sym", ctypes.c_void_p),
+        ("first", ctypes.c_void_p),
+        ("links", ctypes.c_void_p),
+        ("wrap", ctypes.c_int32 * 2),
+    ]
+
+
+LBM_TILE_PERIODIC, LBM_TILE_WALLS, LBM_TILE_LINKS = 0, 1, 2
+
+
 class Instance(ctypes.Structure):
     """lbm_instance of include/lbm_gb300.h (one member of an ensemble)."""
 
@@ -434,7 +462,8 @@ class SchemeModule:
         self.compute = compute
         text = source_obj.module_source(storage, compute)
         deps = "".join(open(os.path.join(CSRC, f)).read()
-                       for f in ("lbm_common.cuh", "lbm_mlp.cuh", "lbm_tc.cuh", "scheme_kernels.cuh"))
+                       for f in ("lbm_common.cuh", "lbm_mlp.cuh", "lbm_tc.cuh", "scheme_kernels.cuh",
+                                 "tile_steps.cuh"))
         deps += open(os.path.join(INCLUDE, "lbm_gb300.h")).read()
         flags = list(getattr(source_obj, "nvcc_flags", []))
         key = hashlib.sha256((text + deps + " ".join(ARCH_FLAGS + flags)).encode()).hexdigest()[:20]
@@ -472,6 +501,9 @@ class SchemeModule:
         _sig(lib, "lbm_one_time_step", I32, [P, P, LP, P, P])
         _sig(lib, "lbm_one_time_step_periodic", I32, [P, P, LP, P, P])
         _sig(lib, "lbm_one_time_step_walls", I32, [P, P, LP, P, P, P, P])
+        _sig(lib, "lbm_scheme_multi_step_plan", I32, [LP, I32, I32, I32, ctypes.POINTER(TilePlan)])
+        _sig(lib, "lbm_scheme_multi_step", I32, [P, P, LP, P, ctypes.POINTER(TilePlan), I32, I32,
+                                                 ctypes.POINTER(TileBoundary), P])
         _sig(lib, "lbm_transport", I32, [P, P, LP, P])
         _sig(lib, "lbm_f2m", I32, [P, LP, P, LP, P])
         _sig(lib, "lbm_f2m_conserved", I32, [P, LP, P, LP, P])

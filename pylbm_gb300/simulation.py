@@ -29,8 +29,8 @@ import numpy as np
 import sympy as sp
 
 from . import runtime
-from .boundary import Boundary, batch_entries, box_wall_table, observed_ghost_copies
-from .codegen import SchemeSource
+from .boundary import Boundary, batch_entries, box_wall_table, observed_ghost_copies, tile_links
+from .codegen import SchemeSource, opposite_populations
 from .domain import Domain
 from .scheme import Scheme
 
@@ -230,6 +230,10 @@ class Simulation:
         # launch, FP16 0.249 against 0.256, BF16 0.250 against 0.253)
         self.fold_walls = True
         self._walls = None          # (constants nv x 27, opposite populations) of lbm_one_time_step_walls
+        self.multi_step = True      # run() advances several steps per launch where the lattice allows it
+        self._multi = {}            # (lbm_tile_plan, lbm_tile_boundary) by mode
+        self._multi_steps = 0       # steps advanced that way
+        self._batch_entries = None  # links of the batched boundary launch, FP32 form, for the tiles
         self._graph = None
         self._graph_key = None
         self._need_init = True
@@ -382,6 +386,9 @@ class Simulation:
         self._upload_ghost()
         self._bc_batch = self._batch_table()
         self._walls = self._wall_table()
+        self._multi = {}
+        if self._multi_mode() == runtime.LBM_TILE_LINKS:
+            self._multi_plan(runtime.LBM_TILE_LINKS)  # with the other lists, not in the first run
 
     def _wall_table(self):
         """Constants of the bounce-back box walls folded into the step, or None."""
@@ -462,6 +469,7 @@ class Simulation:
         and stores its result (the value the copy would have moved)."""
         self._batch_rhs = []   # (device array, method index, host builder) refreshed with time_bc
         self._batch_bufs = []  # device lists made for the table
+        self._batch_entries = None
         g = self._ghost
         ghost = (g["istore_host"], g["iload_host"]) if g is not None else None
         ext = [self.scheme.nv] + [n + 2 * int(h) for n, h in zip(self.domain.shape_in, self.domain.halo)]
@@ -472,6 +480,7 @@ class Simulation:
         if g is not None:
             g["joined"] = joined
         rows = []
+        tiled = []
         # shifted storage: the links compute in FP32 on the stored deviations,
         # with the shifts folded into one per-link constant (LBM_BC_FLOAT_FORM)
         float_form = self.storage != "float64"
@@ -514,6 +523,8 @@ class Simulation:
                 if dist_host is not None:
                     dist = self._device_array(np.ascontiguousarray(dist_host, dtype=np.float32), 4)
                     self._batch_bufs.append(dist)
+                tiled.append({"kind": e["kind"], "iload": e["iload"], "istore": e["istore"], "rhs": rhs_of(m),
+                              "dist": dist_host})
             else:
                 rhs, dist = dev["rhs"], dev.get("dist")
                 if links is not None:
@@ -532,6 +543,8 @@ class Simulation:
             if g is not None:
                 g["joined"] = False
             return None
+        if float_form and (g is None or g["joined"]):
+            self._batch_entries = tiled
         return self._table(rows)
 
     def _flat_slots(self, rows):
@@ -839,20 +852,100 @@ class Simulation:
         self._graph = None
         self._graph_key = None
 
-    def _capture(self, prm):
-        """Capture two steps (F -> Fnew -> F) into one executable graph."""
+    def _multi_mode(self):
+        """Mode of the launches that advance several steps, or None where
+        steps go one by one."""
+        if not self.multi_step or self.dim != 2 or self.compute != "float32" or getattr(self, "closure", None) is not None:
+            return None
+        if self.periodic:
+            return runtime.LBM_TILE_PERIODIC
+        if self._folded():
+            return runtime.LBM_TILE_WALLS
+        if self._bc_batch is not None and self.batch_boundary and self._batch_entries is not None and not self._full_halo:
+            return runtime.LBM_TILE_LINKS
+        return None
+
+    def _multi_plan(self, mode, shape=-1, margin=0):
+        """(lbm_tile_plan, lbm_tile_boundary) of multi-step launches, or None
+        where the lattice or its links take single steps; kept by mode (a shape
+        and margin replace those of the rule)."""
+        if mode in self._multi and shape < 0:
+            return self._multi[mode]
+        plan, bnd = runtime.TilePlan(), runtime.TileBoundary()
+        self.module.call(self.module.lib.lbm_scheme_multi_step_plan(ctypes.byref(self._lat), mode, shape, margin,
+                                                                    ctypes.byref(plan)))
+        multi = (plan, bnd) if plan.shape >= 0 else None
+        if multi is not None and mode == runtime.LBM_TILE_WALLS:
+            table, sym = self._walls
+            bnd.table, bnd.sym = table.ctypes.data, sym.ctypes.data
+        elif multi is not None and mode == runtime.LBM_TILE_LINKS:
+            wrap = [int(self.domain.box_label[2 * d]) == -1 for d in range(2)]
+            ghost = (self._ghost["istore_host"], self._ghost["iload_host"]) if self._ghost is not None else None
+            vel = self.scheme.stencil.get_all_velocities()
+            lists = tile_links(self._batch_entries, ghost, self.domain.shape_in, self.domain.halo, wrap, vel,
+                               opposite_populations(vel), plan)
+            if lists is None:
+                multi = None
+            else:
+                first, links = (self._device_array(a, 4) for a in lists)
+                self._batch_bufs += [first, links]
+                bnd.first, bnd.links = first.ptr, links.ptr
+                bnd.wrap[0], bnd.wrap[1] = int(wrap[0]), int(wrap[1])
+        self._multi[mode] = multi
+        return multi
+
+    def _run_multi(self, nsteps, prm):
+        """Up to ``nsteps`` steps in launches of several; returns their number.
+
+        An even number of steps in an even number of launches, so that the
+        populations end in the buffer in which single steps would leave them;
+        with boundary links two or three single steps are left to the caller,
+        which leave the ghost populations as single steps do."""
+        mode = self._multi_mode()
+        if mode is None:
+            return 0
+        steps = (nsteps - 2 if mode == runtime.LBM_TILE_LINKS else nsteps) // 2 * 2
+        multi = self._multi_plan(mode) if steps >= 4 else None
+        if multi is None:
+            return 0
+        # sixteen launches to a graph once the run is long enough to repay the
+        # capture (between graph nodes a launch costs 1.5 us less)
+        unit = 16 * multi[0].margin
+        key = (self._F.ptr, self._Fnew.ptr, tuple(prm), mode, multi[0].shape, multi[0].margin)
+        self._multi_steps += steps
+        if steps >= unit and self._graph_key != key and self._multi_steps >= 2 * unit:
+            self._capture(lambda: self._enqueue_multi(mode, multi, prm, unit), key)
+        done = 0
+        if self._graph_key == key:
+            for _ in range(steps // unit):
+                runtime.check(self._core.lbm_graph_launch(self._graph, self._stream))
+            done = steps // unit * unit
+        if steps > done:
+            self._enqueue_multi(mode, multi, prm, steps - done)
+        return steps
+
+    def _enqueue_multi(self, mode, multi, prm, steps):
+        plan, bnd = multi
+        self.module.call(self.module.lib.lbm_scheme_multi_step(
+            self._F.handle, self._Fnew.handle, ctypes.byref(self._lat), prm.ctypes.data_as(ctypes.c_void_p),
+            ctypes.byref(plan), steps, mode, ctypes.byref(bnd), self._stream))
+
+    def _enqueue_two_steps(self, prm):
+        self._enqueue_step(self._F, self._Fnew, prm)
+        self._enqueue_step(self._Fnew, self._F, prm)
+
+    def _capture(self, enqueue, key):
+        """Capture steps that leave the populations in F into one executable graph."""
         self._drop_graph()
         runtime.check(self._core.lbm_graph_begin(self._stream))
         try:
-            self._enqueue_step(self._F, self._Fnew, prm)
-            self._enqueue_step(self._Fnew, self._F, prm)
+            enqueue()
         finally:
             g = ctypes.c_void_p()
             rc = self._core.lbm_graph_end(self._stream, ctypes.byref(g))
         runtime.check(rc)
         self._graph = g
-        self._graph_key = (self._F.ptr, self._Fnew.ptr, tuple(prm), self._folded(), self.batch_boundary,
-                           getattr(self, "closure_kernel", None))
+        self._graph_key = key
 
     def run(self, nsteps, graph=True):
         """Advance ``nsteps`` time steps (same result as calling one_time_step)."""
@@ -865,18 +958,23 @@ class Simulation:
                 self.one_time_step()
             return
         prm = self._prm()
-        if self._graph_key != (self._F.ptr, self._Fnew.ptr, tuple(prm), self._folded(), self.batch_boundary,
-                               getattr(self, "closure_kernel", None)):
-            self._capture(prm)
-        for _ in range(nsteps // 2):
+        many = self._run_multi(nsteps, prm)
+        pairs = 0
+        if not many:
+            key = (self._F.ptr, self._Fnew.ptr, tuple(prm), self._folded(), self.batch_boundary,
+                   getattr(self, "closure_kernel", None))
+            if self._graph_key != key:
+                self._capture(lambda: self._enqueue_two_steps(prm), key)
+            pairs = nsteps // 2
+        for _ in range(pairs):
             runtime.check(self._core.lbm_graph_launch(self._graph, self._stream))
+        for _ in range(many + 2 * pairs):
             self.t += self.dt
-            self.t += self.dt
-            self.nt += 2
+        self.nt += many + 2 * pairs
         self._update_m = True
         self._eq_pending = False
         self._m_cache = {}
-        if nsteps % 2:
+        for _ in range(nsteps - many - 2 * pairs):
             self.one_time_step()
 
     def synchronize(self):

@@ -1,0 +1,80 @@
+"""Several steps in one launch (lbm_scheme_multi_step) against single steps.
+
+The region kernel holds the values in the storage type and runs the same
+generated collision, so the populations, ghost layer included, must be those
+of single launches bit for bit: periodic grids (smaller than a region, odd,
+wider than one), box walls, and boundary links of every method on obstacles,
+for each region shape and for the rule's choice.
+"""
+import numpy as np
+import pytest
+
+from pylbm_gb300 import Simulation
+from pylbm_gb300 import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+FLOWS = {
+    "shear8": lambda: W.shear_layer(n=8),
+    "shear97": lambda: W.shear_layer(n=97),
+    "shear128": lambda: W.shear_layer(n=128),
+    "cavity33": lambda: W.cavity(n=33),
+    "cavity96": lambda: W.cavity(n=96),
+    "disc": lambda: W.cylinder(nx=131, ny=48, radius=3, center=(26, 25), re=18.75),
+    "karman": lambda: W.karman(dx=1.0 / 64),
+}
+C0 = {"disc": [1.0, 0.05, 0.0], "karman": [1.0, 0.05, 0.0]}
+# shape and margin; the last is the rule's choice
+PLANS = [(0, 5), (0, 10), (1, 6), (2, 3), (2, 8), (-1, 0)]
+
+
+def _populations(sim):
+    return np.array([sim.F_halo[k] for k in range(sim.scheme.nv)])
+
+
+@pytest.mark.parametrize("flow, dtype", [(f, "float32") for f in FLOWS] +
+                         [("shear97", "float16"), ("shear128", "bfloat16"), ("cavity33", "float16")])
+def test_multi_step_equals_single_steps(flow, dtype):
+    def make():
+        return Simulation(FLOWS[flow](), dtype=dtype, c0=C0.get(flow, [1.0, 0.0, 0.0]))
+
+    single = make()
+    single.multi_step = False
+    single.run(23)
+    ref = _populations(single)
+    single.free()
+    assert np.all(np.isfinite(ref))
+    for shape, margin in PLANS:
+        sim = make()
+        mode = sim._multi_mode()
+        assert mode is not None
+        assert sim._multi_plan(mode, shape, margin) is not None
+        sim.run(23)
+        assert sim.nt == 23
+        assert np.array_equal(_populations(sim), ref), (shape, margin)
+        sim.free()
+
+
+def test_captured_launches_continue_the_run():
+    runs = []
+    for multi in (True, False):
+        sim = Simulation(W.shear_layer(n=97), dtype="float32", c0=[1.0, 0.0, 0.0])
+        sim.multi_step = multi
+        for steps in (500, 3, 700, 2):
+            sim.run(steps)
+        assert sim.nt == 1205
+        runs.append(_populations(sim))
+        sim.free()
+    assert np.array_equal(*runs)
+
+
+def test_single_steps_remain_where_they_must():
+    sim = Simulation(W.cavity(n=32))   # FP64
+    assert sim._multi_mode() is None
+    sim.free()
+    sim = Simulation(W.karman(dx=1.0 / 64), dtype="float32", c0=C0["karman"], halo="full")
+    assert sim._multi_mode() is None
+    sim.free()
+    sim = Simulation(W.tgv3d(n=16), dtype="float32")
+    assert sim._multi_mode() is None
+    sim.free()
