@@ -482,8 +482,8 @@ int lbm_one_time_step_walls(const void* f, void* fnew, const lbm_lattice* lat, c
  * with `margin`, the most steps of a launch.  plan->shape is -1 where single
  * steps are to be used (another dimension, reach, storage or size).
  *
- * lbm_scheme_multi_step advances `steps` steps (even) from f in an even
- * number of launches between f and fnew, so that the result lies in f.
+ * lbm_scheme_multi_step advances `steps` steps (a multiple of granule) from f
+ * in an even number of launches between f and fnew, so that the result lies in f.
  * No reference counterpart. */
 enum { LBM_TILE_PERIODIC = 0, LBM_TILE_WALLS = 1, LBM_TILE_LINKS = 2 };
 
@@ -494,6 +494,8 @@ typedef struct lbm_tile_plan {
   int32_t tiles[2];  /* blocks along each axis */
   int32_t pitch;     /* elements between rows of the region in shared memory */
   int32_t plane;     /* elements between populations there */
+  int32_t planes;    /* 3D: output planes of a block along the outermost axis */
+  int32_t granule;   /* steps come in multiples of this */
 } lbm_tile_plan;
 
 /* One boundary link of one tile: element offsets in the region of the slot it

@@ -727,7 +727,8 @@ class SchemeSource:
         return (f"#define LBM_STORAGE {ctypes_[storage]}\n"
                 f"#define LBM_COMPUTE {ctypes_[compute]}\n"
                 + ("#define LBM_PAIRS 1\n" if pairs else "")
-                + ("#define LBM_FLOAT_COMPUTE 1\n" if compute == "float32" else "") +
+                + ("#define LBM_FLOAT_COMPUTE 1\n" if compute == "float32" else "")
+                + ("#define LBM_PLANE_STEPS 1\n" if storage == "float32" and not self.absolute_collide else "") +
                 "#include \"lbm_common.cuh\"\n"
                 "using lbm::lbm_fma;\n"
                 "template <typename R> __device__ __forceinline__ R lbm_sqrt(R x) { return sqrt(x); }\n"

@@ -1,0 +1,278 @@
+// Two time steps of a 3D lattice in one launch (included by
+// scheme_kernels.cuh inside lbm_scheme).
+//
+// One step at a time FP32 D3Q19 runs at the copy bandwidth (152 bytes a node;
+// 256^3: 0.389 ms of a 0.382 ms floor), so only less traffic makes it faster:
+// a block walks along the outermost axis over a column of the grid, computes
+// the first step of one plane after the other from global memory, keeps it in
+// shared memory and finishes the second step of the plane behind, so that two
+// steps read and write the populations once.
+//
+// Output plane q - 1 needs, of the first step's populations, those moving
+// down (v0 = -1) of plane q, the level ones (v0 = 0) of plane q - 1 and those
+// moving up (v0 = +1) of plane q - 2.  These 2 x level + 3 x up + 1 x down
+// planes are all that is kept, each value exactly until the one node that
+// pulls it has read it: the node then writes its own next values into the
+// slots it has read, so one barrier a plane suffices.  In detail, with x the
+// position in the column's cross-section and k' opposite to k:
+//   level  two buffers by the parity of the plane, each filled in turn as
+//          f_k(x) -> (k, x) and as f_k(x) -> (k', x + v_k)
+//   up     f_k(x) -> (k, x) in buffer q mod 4
+//   down   f_k(x) -> (k', x + v_k) in buffer (q + 1) mod 4, whose slots held
+//          the up values of plane q - 3 that the same nodes have just read
+// A thread owns one position of the cross-section for the whole walk, rows
+// laid end to end over the threads, so that no lane is idle for the width's
+// sake and every shared access is one word per lane along consecutive words.
+// One block of 640 threads an SM leaves 102 registers: enough to hold the next
+// plane's 19 loads in flight during the second step, which is worth more than
+// occupancy (two blocks of 512 threads without it: 487 us a step at 256^3).
+//
+// Measured, D3Q19 FP32, us a step before -> after: 256^3 385 -> 264, 192^3
+// 163 -> 114, 128^3 53 -> 37, 96^3 24.5 -> 17.8; lid-driven cube 131^3
+// 67.7 -> 50.2.  At 256^3 issue slots are 60 % busy and HBM 55 %.
+// FP32 storage with the plain collision only: 16-bit storage moves half the
+// bytes and its two-node step is bound by instructions as this one is (D3Q19
+// FP16 192^3: 102 us a step), and a collision of more arithmetic (relative
+// velocity, sources) would repeat it at the columns' borders.
+#if LBM_DIM == 3 && LBM_VMAX == 1 && defined(LBM_FOR_EACH_AA) && defined(LBM_PLANE_STEPS) && LBM_Q <= 19
+#define LBM_HAS_PLANE_STEPS 1
+
+struct PlaneArgs {
+  int n[3];
+  int stride0, stride1;  // elements
+  int vstride;
+  int base;              // element offset of interior node (0, 0, 0) of population 0
+  int out1, out2;        // output rows and columns of a column of the grid
+  int planes;            // output planes of a block
+  R prm[kPrm];
+};
+
+constexpr int kPlaneThreads = 640;
+constexpr int kPlaneSlack = 72;  // a row and a place: what x + v_k reaches beyond the cross-section
+constexpr int kPlaneSpan = kPlaneThreads + 2 * kPlaneSlack;
+
+__host__ __device__ constexpr int axis0_velocity(int k) {
+#define LBM_AXIS0(j, vx, vy, vz, jo) (k == (j)) ? (vx) :
+  return LBM_FOR_EACH_AA(LBM_AXIS0) 0;
+#undef LBM_AXIS0
+}
+// number of populations before k with the axis-0 velocity of k
+__host__ __device__ constexpr int index_in_group(int k) {
+  int n = 0;
+  for (int j = 0; j < k; ++j) n += axis0_velocity(j) == axis0_velocity(k);
+  return n;
+}
+__host__ __device__ constexpr int group_size(int v0) {
+  int n = 0;
+  for (int j = 0; j < LBM_Q; ++j) n += axis0_velocity(j) == v0;
+  return n;
+}
+constexpr int kLevel = group_size(0), kUp = group_size(1);
+constexpr int kKept = 2 * kLevel + 4 * kUp;  // sub-arrays; then two times kUp of kept values (walls)
+template <bool kWalls>
+constexpr size_t kPlaneBytes = (size_t)(kKept + (kWalls ? 2 * kUp : 0)) * kPlaneSpan * sizeof(S);
+
+// slot of the first step's population k of a plane of phase J (its number mod
+// 4): sub-array and displacement from x
+template <int J, int k, int vx, int vy, int vz, int ko>
+struct PlaneSlot {
+  static constexpr bool kLevelSwapped = (J >> 1) & 1;
+  static constexpr bool kSwapped = vx < 0 || (vx == 0 && kLevelSwapped);
+  static constexpr int kArray = vx == 0 ? (J & 1) * kLevel + index_in_group(kSwapped ? ko : k)
+                                : vx > 0 ? 2 * kLevel + J * kUp + index_in_group(k)
+                                         : 2 * kLevel + ((J + 1) & 3) * kUp + index_in_group(ko);
+  // where x finds f_k(x - v_k), and where it puts f_k(x)
+  __device__ __forceinline__ static int get(int pitch) { return kArray * kPlaneSpan - (kSwapped ? 0 : vy * pitch + vz); }
+  __device__ __forceinline__ static int put(int pitch) { return kArray * kPlaneSpan + (kSwapped ? vy * pitch + vz : 0); }
+};
+
+struct PlaneThread {
+  unsigned row[3], col[3];  // byte offsets of the rows and columns at -1, 0, +1 of this position, wrapped
+  int pitch;
+  bool active, inside;      // in the cross-section; in its output part
+  // walls: shares of the constants' index where a source lies below or above
+  // the grid along axes 1 and 2 (0 away from the faces)
+  int below1, above1, below2, above2;
+  bool side;                // walls: a lane of the warp lies at one of these faces
+};
+
+__device__ __forceinline__ int plane_wrap(int c, int n) {
+  if (c < 0) c += n;
+  if (c >= n) c -= n;
+  return c;
+}
+
+// uniform pointer plus a lane's 32-bit byte offset: one address register per load
+template <typename T>
+__device__ __forceinline__ T* plane_at(T* base, unsigned offset) {
+  return reinterpret_cast<T*>(reinterpret_cast<uintptr_t>(base) + offset);
+}
+
+// walls the source of population k of a node of plane q lies beyond, as the
+// index 9 (o0 + 1) + 3 (o1 + 1) + (o2 + 1) of their constants (13: none)
+__device__ __forceinline__ int plane_sig(const PlaneArgs& a, const PlaneThread& t, int q, int vx, int vy, int vz) {
+  return 13 + 9 * wall_off(vx, q == 0, q == a.n[0] - 1) + (vy == 0 ? 0 : vy > 0 ? t.below1 : t.above1) +
+         (vz == 0 ? 0 : vz > 0 ? t.below2 : t.above2);
+}
+
+// what the first step of plane q (grid coordinate) pulls; beyond a wall the
+// opposite population of the node itself
+template <bool kWalls>
+__device__ __forceinline__ void plane_pull(const S* __restrict__ f, const PlaneArgs& a, const PlaneThread& t, int q,
+                                           R (&g)[LBM_Q]) {
+  if (!t.active || (kWalls && (q < 0 || q >= a.n[0]))) return;
+  const int q0 = plane_wrap(q, a.n[0]);
+  const S* below = f + (long long)(plane_wrap(q0 - 1, a.n[0])) * a.stride0;
+  const S* level = f + (long long)q0 * a.stride0;
+  const S* above = f + (long long)(plane_wrap(q0 + 1, a.n[0])) * a.stride0;
+  if (kWalls && (t.side || q == 0 || q == a.n[0] - 1)) {
+#define LBM_PLANE_PULL_WALL(k, vx, vy, vz, ko)                                                        \
+  {                                                                                                   \
+    const bool out = plane_sig(a, t, q, vx, vy, vz) != 13;                                            \
+    const S* from = ((vx) > 0 ? below : (vx) < 0 ? above : level) + (long long)(k) * a.vstride;       \
+    g[k] = (R)Store<S>::load(plane_at(out ? level + (long long)(ko) * a.vstride : from,               \
+                                      out ? t.row[1] + t.col[1] : t.row[1 - (vy)] + t.col[1 - (vz)])); \
+  }
+    LBM_FOR_EACH_AA(LBM_PLANE_PULL_WALL)
+#undef LBM_PLANE_PULL_WALL
+    return;
+  }
+#define LBM_PLANE_PULL(k, vx, vy, vz, ko)                                                                       \
+  g[k] = (R)Store<S>::load(plane_at(((vx) > 0 ? below : (vx) < 0 ? above : level) + (long long)(k) * a.vstride, \
+                                    t.row[1 - (vy)] + t.col[1 - (vz)]));
+  LBM_FOR_EACH_AA(LBM_PLANE_PULL)
+#undef LBM_PLANE_PULL
+}
+
+// the first step of plane q from what it pulls, into the slots of its phase.
+// With walls: a level population that leaves the grid stays in the node's own
+// slot (k, x), and the down populations are kept for one plane more, for the
+// up populations that come back from a wall.
+template <int J, bool kWalls>
+__device__ __forceinline__ void plane_first(S* __restrict__ p, const PlaneArgs& a, const PlaneThread& t,
+                                            const WallArgs& w, int q, R (&g)[LBM_Q]) {
+  if (!t.active || (kWalls && (q < 0 || q >= a.n[0]))) return;
+  const bool walls = kWalls && (t.side || q == 0 || q == a.n[0] - 1);
+  if (walls) {
+    // selects, not branches: a face has one lane in a row of them
+#define LBM_PLANE_WALL(k, vx, vy, vz, ko)               \
+  {                                                     \
+    const int sig = plane_sig(a, t, q, vx, vy, vz);     \
+    const R back = through_storage(g[k] + w.c[k][sig]); \
+    g[k] = sig != 13 ? back : g[k];                     \
+  }
+    LBM_FOR_EACH_AA(LBM_PLANE_WALL)
+#undef LBM_PLANE_WALL
+  }
+  lbm_collide<R>(g, a.prm);
+  if (walls) {
+#define LBM_PLANE_PUT_WALL(k, vx, vy, vz, ko)                                                                      \
+  {                                                                                                                \
+    using Slot = PlaneSlot<J, k, vx, vy, vz, ko>;                                                                  \
+    constexpr int kOwn = ((J & 1) * kLevel + index_in_group(k)) * kPlaneSpan;                                      \
+    constexpr int kKeep = (kKept + (J & 1) * kUp + index_in_group(k)) * kPlaneSpan;                                \
+    const bool stay = (vx) == 0 && Slot::kSwapped &&                                                               \
+                      (((vy) < 0 && t.below1) || ((vy) > 0 && t.above1) || ((vz) < 0 && t.below2) ||               \
+                       ((vz) > 0 && t.above2));                                                                    \
+    Store<S>::store(p + (stay ? kOwn : Slot::put(t.pitch)), g[k]);                                                 \
+    if ((vx) < 0) Store<S>::store(p + kKeep, g[k]);                                                                \
+  }
+    LBM_FOR_EACH_AA(LBM_PLANE_PUT_WALL)
+#undef LBM_PLANE_PUT_WALL
+    return;
+  }
+#define LBM_PLANE_PUT(k, vx, vy, vz, ko) Store<S>::store(p + PlaneSlot<J, k, vx, vy, vz, ko>::put(t.pitch), g[k]);
+  LBM_FOR_EACH_AA(LBM_PLANE_PUT)
+#undef LBM_PLANE_PUT
+}
+
+// second step of plane q - 1, after the first of plane q
+template <int J, bool kWalls>
+__device__ __forceinline__ void plane_second(S* __restrict__ fnew, const S* __restrict__ p, const PlaneArgs& a,
+                                             const PlaneThread& t, const WallArgs& w, int q) {
+  if (!t.inside) return;
+  R g[LBM_Q];
+#define LBM_PLANE_GET(k, vx, vy, vz, ko) \
+  g[k] = SharedValue<S>::get(p + PlaneSlot<(J + 4 - ((vx) + 1)) & 3, k, vx, vy, vz, ko>::get(t.pitch));
+  LBM_FOR_EACH_AA(LBM_PLANE_GET)
+#undef LBM_PLANE_GET
+  if (kWalls && (t.side || q == 1 || q == a.n[0])) {
+    // f_k'(x) of plane q - 1: a level or up population in its own slot, a down one as kept
+#define LBM_PLANE_BACK(k, vx, vy, vz, ko)                                                             \
+  {                                                                                                   \
+    constexpr int kP = (J + 3) & 3; /* phase of plane q - 1 */                                        \
+    constexpr int kFrom = (vx) == 0  ? (kP & 1) * kLevel + index_in_group(ko)                         \
+                          : (vx) > 0 ? kKept + (kP & 1) * kUp + index_in_group(ko)                    \
+                                     : 2 * kLevel + kP * kUp + index_in_group(ko);                    \
+    const int sig = plane_sig(a, t, q - 1, vx, vy, vz);                                               \
+    const R back = through_storage(SharedValue<S>::get(p + kFrom * kPlaneSpan) + w.c[k][sig]);        \
+    g[k] = sig != 13 ? back : g[k];                                                                   \
+  }
+    LBM_FOR_EACH_AA(LBM_PLANE_BACK)
+#undef LBM_PLANE_BACK
+  }
+  lbm_collide<R>(g, a.prm);
+  S* d = fnew + (long long)(q - 1) * a.stride0;
+#pragma unroll
+  for (int k = 0; k < LBM_Q; ++k) Store<S>::store(plane_at(d + (long long)k * a.vstride, t.row[1] + t.col[1]), g[k]);
+}
+
+template <bool kWalls>
+__global__ void __launch_bounds__(kPlaneThreads, 1) k_two_steps(const S* __restrict__ f, S* __restrict__ fnew,
+                                                              const __grid_constant__ PlaneArgs a,
+                                                              const __grid_constant__ WallArgs w) {
+  extern __shared__ __align__(16) unsigned char plane_smem[];
+  __shared__ uint64_t done;  // the first step of a plane, by warps
+  PlaneThread t;
+  t.pitch = a.out2 + 2;
+  const int r = threadIdx.x / t.pitch, c = threadIdx.x - r * t.pitch;
+  const int i1 = (int)blockIdx.y * a.out1 - 1 + r, i2 = (int)blockIdx.x * a.out2 - 1 + c;
+  t.active = r < a.out1 + 2 && i1 <= a.n[1] && i2 <= a.n[2];
+  if (kWalls) t.active = t.active && i1 >= 0 && i1 < a.n[1] && i2 >= 0 && i2 < a.n[2];
+  t.inside = t.active && r >= 1 && r <= a.out1 && c >= 1 && c <= a.out2 && i1 < a.n[1] && i2 < a.n[2];
+  t.below1 = i1 == 0 ? -3 : 0;
+  t.above1 = i1 == a.n[1] - 1 ? 3 : 0;
+  t.below2 = i2 == 0 ? -1 : 0;
+  t.above2 = i2 == a.n[2] - 1 ? 1 : 0;
+  t.side = __any_sync(0xffffffffu, (t.below1 | t.above1 | t.below2 | t.above2) != 0);
+#pragma unroll
+  for (int s = 0; s < 3; ++s) {
+    t.row[s] = (a.base + plane_wrap(plane_wrap(i1, a.n[1]) + s - 1, a.n[1]) * a.stride1) * (unsigned)sizeof(S);
+    t.col[s] = plane_wrap(plane_wrap(i2, a.n[2]) + s - 1, a.n[2]) * (unsigned)sizeof(S);
+  }
+  S* p = reinterpret_cast<S*>(plane_smem) + kPlaneSlack + threadIdx.x;
+  if (threadIdx.x == 0) {
+    lbm::mbar_init(&done, kPlaneThreads / 32);
+    lbm::mbar_init_fence();
+  }
+  __syncthreads();
+  uint32_t parity = 0;
+  const int begin = (int)blockIdx.z * a.planes, end = min(begin + a.planes, a.n[0]);
+  int q = begin - 1;
+  R g[LBM_Q];
+  plane_pull<kWalls>(f, a, t, q, g);
+  // A warp announces its part of a first step, sets off the loads of the next
+  // plane and only then waits for the other warps: the loads are in flight
+  // during the second step, and the wait (bounded) rarely stalls.
+#define LBM_PLANE_PHASE(J)                                       \
+  plane_first<J, kWalls>(p, a, t, w, q, g);                       \
+  __syncwarp();                                                  \
+  if ((threadIdx.x & 31) == 0) lbm::mbar_arrive(&done);          \
+  if (q < end) plane_pull<kWalls>(f, a, t, q + 1, g);            \
+  if (!lbm::mbar_wait(&done, parity)) {                          \
+    if ((threadIdx.x & 31) == 0) atomicAdd(&lbm_wait_timeouts, 1u); \
+    break;                                                       \
+  }                                                              \
+  parity ^= 1;                                                   \
+  if (q > begin) plane_second<J, kWalls>(fnew, p, a, t, w, q);      \
+  if (++q > end) break;
+#pragma unroll 1
+  while (true) {
+    LBM_PLANE_PHASE(0)
+    LBM_PLANE_PHASE(1)
+    LBM_PLANE_PHASE(2)
+    LBM_PLANE_PHASE(3)
+  }
+#undef LBM_PLANE_PHASE
+}
+#endif

@@ -1278,6 +1278,7 @@ __global__ void __launch_bounds__(LBM_BLOCK) k_source_term(double* __restrict__ 
 }
 
 #include "tile_steps.cuh"
+#include "plane_steps.cuh"
 
 // ------------------------------------------------------------------ host
 // need_halo: the stencil reach in ghost layers, for the kernels that pull
@@ -1880,6 +1881,71 @@ inline void tile_rule(const lbm_lattice& lat, int& shape, int& margin) {
 }  // namespace lbm_scheme
 #endif
 
+#if LBM_HAS_PLANE_STEPS
+namespace lbm_scheme {
+
+template <bool kWalls>
+static int plane_grant(const char* who) {
+  static bool done[64];
+  int dev = 0;
+  int rc = lbm::cuda_check(cudaGetDevice(&dev), who);
+  if (rc || (dev >= 0 && dev < 64 && done[dev])) return rc;
+  rc = lbm::cuda_check(cudaFuncSetAttribute(k_two_steps<kWalls>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                            (int)kPlaneBytes<kWalls>),
+                       who);
+  if (!rc && dev >= 0 && dev < 64) done[dev] = true;
+  return rc;
+}
+
+// columns and planes of the two-step walk
+inline void plane_rule(const lbm_lattice& lat, bool walls, int shape, lbm_tile_plan& plan) {
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1) {
+    (void)cudaGetLastError();
+    sms = 152;
+  }
+  const int n0 = lat.n[0], n1 = lat.n[1], n2 = lat.n[2];
+  // Expected microseconds: two single steps, 2.8 and the traffic at 6.5 TB/s
+  // each; a two-step launch, 2.5 and 2 more a wave, for every plane of a block
+  // 0.35 and 0.045 a warp and step (19 populations; short rows, read in part
+  // sectors, cost more, and so do rows that end at walls: with one wave the
+  // blocks at the walls set the time, with several they are shared out).  D3Q19 FP32 at 24^3 to 256^3 keeps to
+  // it within 12 %.
+  double best = shape >= 0 ? 1e30 : (walls ? 0.90 : 0.97) * 2.0 * (2.8 + (double)n0 * n1 * n2 * 2 * LBM_Q * sizeof(S) / 6.5e6);
+  const double warp_us = 0.045 * LBM_Q / 19;
+  for (int t2 = (n2 + kPlaneSlack - 4) / (kPlaneSlack - 3); t2 <= n2; ++t2) {
+    const int o2 = (n2 + t2 - 1) / t2, most = kPlaneThreads / (o2 + 2) - 2;
+    if (o2 < 6 || (o2 < 20 && t2 > 1)) break;  // short rows are read in part sectors
+    for (int t1 = (n1 + most - 1) / most; t1 <= n1; ++t1) {
+      const int o1 = (n1 + t1 - 1) / t1;
+      if (o1 < 4) break;
+      const double first = ((o1 + 2) * (o2 + 2) + 31) / 32, second = (o1 * (o2 + 2) + 31) / 32 + 1;
+      for (int t0 = 1; t0 <= (n0 + 3) / 4; ++t0) {
+        const int planes = (n0 + t0 - 1) / t0;
+        if (shape >= 0 && planes != shape) continue;
+        const double waves = (double)(((long long)t0 * t1 * t2 + sms - 1) / sms);
+        const double warps = (planes + 2) * first + planes * second;
+        const double row = !walls ? 1.0 + 3.0 / o2 : waves > 1.0 ? 1.18 * (1.0 + 5.0 / o2) : 1.2 * (1.0 + 6.0 / o2);
+        const double us = 0.5 + waves * (2.0 + (planes + 2) * 0.35 + row * warp_us * warps);
+        if (us >= best) continue;
+        best = us;
+        plan.shape = 0;
+        plan.margin = 2;
+        plan.out[0] = o1;
+        plan.out[1] = o2;
+        plan.tiles[0] = t1;
+        plan.tiles[1] = t2;
+        plan.planes = planes;
+        plan.granule = 4;
+      }
+    }
+  }
+}
+
+}  // namespace lbm_scheme
+#endif
+
 extern "C" int lbm_scheme_multi_step_plan(const lbm_lattice* lat, int32_t mode, int32_t shape, int32_t margin,
                                    lbm_tile_plan* plan) {
   using namespace lbm_scheme;
@@ -1890,7 +1956,8 @@ extern "C" int lbm_scheme_multi_step_plan(const lbm_lattice* lat, int32_t mode, 
   if (mode < 0 || mode > 2) return lbm::fail(LBM_ERR_ARG, "%s: mode %d", who, mode);
   plan->shape = -1;
   plan->margin = 0;
-  plan->out[0] = plan->out[1] = plan->tiles[0] = plan->tiles[1] = plan->pitch = plan->plane = 0;
+  plan->out[0] = plan->out[1] = plan->tiles[0] = plan->tiles[1] = plan->pitch = plan->plane = plan->planes = 0;
+  plan->granule = 2;
 #if LBM_HAS_TILE_STEPS
   if (lat->elements >= (1LL << 31)) return LBM_OK;  // the kernel indexes with 32 bits
   if (shape >= kTileShapes) return lbm::fail(LBM_ERR_ARG, "%s: shape %d", who, shape);
@@ -1915,12 +1982,36 @@ extern "C" int lbm_scheme_multi_step_plan(const lbm_lattice* lat, int32_t mode, 
     plan->plane = Shape::kPlane;
     return (int)LBM_OK;
   });
+#elif LBM_HAS_PLANE_STEPS
+  (void)margin;
+  if (mode != LBM_TILE_LINKS && kPlaneBytes<true> <= 225 * 1024) plane_rule(*lat, mode == LBM_TILE_WALLS, shape, *plan);
+  return LBM_OK;
 #else
   (void)shape;
   (void)margin;
   return LBM_OK;
 #endif
 }
+
+#if LBM_HAS_TILE_STEPS || LBM_HAS_PLANE_STEPS
+// the wall constants of a multi-step launch
+static int tile_walls(const lbm_lattice* lat, const lbm_tile_boundary* b, lbm_scheme::WallArgs& w, const char* who) {
+  using lbm_scheme::R;
+  if (!b || !b->table || !b->sym) return lbm::fail(LBM_ERR_ARG, "%s: NULL boundary", who);
+  for (int d = 0; d < LBM_DIM; ++d)
+    if (lat->halo[d] != 1) return lbm::fail(LBM_ERR_ARG, "%s: halo[%d]=%d, one ghost layer expected", who, d, lat->halo[d]);
+    // the swapped layouts pair the populations as the walls do
+#define LBM_TILE_SYM(k, vx, vy, vz, ko) \
+  if (b->sym[k] != (ko)) return lbm::fail(LBM_ERR_UNSUPPORTED, "%s: sym[%d]=%d", who, (k), b->sym[k]);
+  LBM_FOR_EACH_AA(LBM_TILE_SYM)
+#undef LBM_TILE_SYM
+  for (int k = 0; k < LBM_Q; ++k) {
+    w.sym[k] = b->sym[k];
+    for (int j = 0; j < 27; ++j) w.c[k][j] = (R)b->table[k * 27 + j];
+  }
+  return LBM_OK;
+}
+#endif
 
 extern "C" int lbm_scheme_multi_step(void* f, void* fnew, const lbm_lattice* lat, const double* prm,
                                      const lbm_tile_plan* plan, int32_t steps, int32_t mode,
@@ -1938,8 +2029,7 @@ extern "C" int lbm_scheme_multi_step(void* f, void* fnew, const lbm_lattice* lat
   if (plan->shape < 0 || plan->shape >= kTileShapes || plan->margin < 1 || steps < 2 || steps % 2)
     return lbm::fail(LBM_ERR_ARG, "%s: shape %d, margin %d, %d steps", who, plan->shape, plan->margin, steps);
   const bool walls = mode == LBM_TILE_WALLS, linked = mode == LBM_TILE_LINKS;
-  if ((walls && (!boundary || !boundary->table || !boundary->sym)) ||
-      (linked && (!boundary || !boundary->first || !boundary->links)))
+  if (linked && (!boundary || !boundary->first || !boundary->links))
     return lbm::fail(LBM_ERR_ARG, "%s: NULL boundary", who);
   StepArgs sa = make_step_args(*lat, prm);
   TileArgs a;
@@ -1959,17 +2049,8 @@ extern "C" int lbm_scheme_multi_step(void* f, void* fnew, const lbm_lattice* lat
   for (int i = 0; i < kPrm; ++i) a.prm[i] = sa.prm[i];
   WallArgs w;
   if (walls) {
-    for (int d = 0; d < 2; ++d)
-      if (lat->halo[d] != 1) return lbm::fail(LBM_ERR_ARG, "%s: halo[%d]=%d, one ghost layer expected", who, d, lat->halo[d]);
-    // the swapped layout pairs the populations as the walls do
-#define LBM_TILE_SYM(k, vx, vy, vz, ko) \
-  if (boundary->sym[k] != (ko)) return lbm::fail(LBM_ERR_UNSUPPORTED, "%s: sym[%d]=%d", who, (k), boundary->sym[k]);
-    LBM_FOR_EACH_AA(LBM_TILE_SYM)
-#undef LBM_TILE_SYM
-    for (int k = 0; k < LBM_Q; ++k) {
-      w.sym[k] = boundary->sym[k];
-      for (int j = 0; j < 27; ++j) w.c[k][j] = (R)boundary->table[k * 27 + j];
-    }
+    rc = tile_walls(lat, boundary, w, who);
+    if (rc) return rc;
   }
   return with_tile_shape(plan->shape, [&](auto tag) {
     using Shape = decltype(tag);
@@ -2001,6 +2082,47 @@ extern "C" int lbm_scheme_multi_step(void* f, void* fnew, const lbm_lattice* lat
     }
     return (int)LBM_OK;
   });
+#elif LBM_HAS_PLANE_STEPS
+  const bool walls = mode == LBM_TILE_WALLS;
+  if (mode == LBM_TILE_LINKS) return lbm::fail(LBM_ERR_UNSUPPORTED, "%s: boundary links in 3D", who);
+  WallArgs w;
+  if (walls) {
+    rc = tile_walls(lat, boundary, w, who);
+    if (rc) return rc;
+  }
+  PlaneArgs a;
+  a.out1 = plan->out[0];
+  a.out2 = plan->out[1];
+  a.planes = plan->planes;
+  if (steps < 4 || steps % 4 || a.out1 < 1 || a.out2 < 1 || a.out2 + 3 > kPlaneSlack || a.planes < 1 ||
+      (a.out1 + 2) * (a.out2 + 2) > kPlaneThreads || (long long)a.out1 * plan->tiles[0] < lat->n[1] ||
+      (long long)a.out2 * plan->tiles[1] < lat->n[2] || plan->tiles[0] > 65535 || lat->stride[0] >= (1LL << 31))
+    return lbm::fail(LBM_ERR_ARG, "%s: %d steps, columns %d x %d, %d planes", who, steps, a.out1, a.out2, a.planes);
+  const StepArgs sa = make_step_args(*lat, prm);
+  for (int d = 0; d < 3; ++d) a.n[d] = lat->n[d];
+  a.stride0 = (int)lat->stride[0];
+  a.stride1 = (int)lat->stride[1];
+  a.vstride = (int)lat->vstride;
+  a.base = (int)(lat->origin + lat->halo[0] * lat->stride[0] + lat->halo[1] * lat->stride[1] + lat->halo[2]);
+  for (int i = 0; i < kPrm; ++i) a.prm[i] = sa.prm[i];
+  rc = walls ? plane_grant<true>(who) : plane_grant<false>(who);
+  if (rc) return rc;
+  const dim3 grid((unsigned)plan->tiles[1], (unsigned)plan->tiles[0],
+                  (unsigned)((lat->n[0] + a.planes - 1) / a.planes));
+  S* from = (S*)f;
+  S* to = (S*)fnew;
+  for (int i = 0; i < steps / 2; ++i) {
+    if (walls)
+      k_two_steps<true><<<grid, kPlaneThreads, kPlaneBytes<true>, (cudaStream_t)stream>>>(from, to, a, w);
+    else
+      k_two_steps<false><<<grid, kPlaneThreads, kPlaneBytes<false>, (cudaStream_t)stream>>>(from, to, a, w);
+    rc = lbm::launch_check(who);
+    if (rc) return rc;
+    S* t = from;
+    from = to;
+    to = t;
+  }
+  return LBM_OK;
 #else
   (void)steps;
   (void)boundary;

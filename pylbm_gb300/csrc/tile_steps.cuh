@@ -25,6 +25,21 @@
 // and the arithmetic is the generated collide of the one-step kernels: the
 // populations after T steps are those of T single launches bit for bit.
 
+// one value of shared memory, in FP32
+template <typename T> struct SharedValue;
+template <> struct SharedValue<double> {
+  __device__ __forceinline__ static double get(const double* p) { return *p; }
+};
+template <> struct SharedValue<float> {
+  __device__ __forceinline__ static float get(const float* p) { return *p; }
+};
+template <> struct SharedValue<__half> {
+  __device__ __forceinline__ static float get(const __half* p) { return __half2float(*p); }
+};
+template <> struct SharedValue<__nv_bfloat16> {
+  __device__ __forceinline__ static float get(const __nv_bfloat16* p) { return __bfloat162float(*p); }
+};
+
 #if LBM_DIM == 2 && LBM_VMAX == 1 && defined(LBM_FOR_EACH_AA) && defined(LBM_FLOAT_COMPUTE) && LBM_Q <= 16
 #define LBM_HAS_TILE_STEPS 1
 
@@ -42,18 +57,6 @@ struct TileArgs {
   const int* first;   // links kernel: first link of every tile, and the total
   const lbm_tile_link* links;
   R prm[kPrm];
-};
-
-// one value of shared memory, in FP32
-template <typename T> struct SharedValue;
-template <> struct SharedValue<float> {
-  __device__ __forceinline__ static float get(const float* p) { return *p; }
-};
-template <> struct SharedValue<__half> {
-  __device__ __forceinline__ static float get(const __half* p) { return __half2float(*p); }
-};
-template <> struct SharedValue<__nv_bfloat16> {
-  __device__ __forceinline__ static float get(const __nv_bfloat16* p) { return __bfloat162float(*p); }
 };
 
 // region shape: kW columns (a multiple of 32) x kH rows, kThreads threads;

@@ -123,6 +123,8 @@ class TilePlan(ctypes.Structure):
         ("tiles", ctypes.c_int32 * 2),
         ("pitch", ctypes.c_int32),
         ("plane", ctypes.c_int32),
+        ("planes", ctypes.c_int32),
+        ("granule", ctypes.c_int32),
     ]
 
 
@@ -463,7 +465,7 @@ class SchemeModule:
         text = source_obj.module_source(storage, compute)
         deps = "".join(open(os.path.join(CSRC, f)).read()
                        for f in ("lbm_common.cuh", "lbm_mlp.cuh", "lbm_tc.cuh", "scheme_kernels.cuh",
-                                 "tile_steps.cuh"))
+                                 "tile_steps.cuh", "plane_steps.cuh"))
         deps += open(os.path.join(INCLUDE, "lbm_gb300.h")).read()
         flags = list(getattr(source_obj, "nvcc_flags", []))
         key = hashlib.sha256((text + deps + " ".join(ARCH_FLAGS + flags)).encode()).hexdigest()[:20]

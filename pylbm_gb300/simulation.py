@@ -855,13 +855,13 @@ class Simulation:
     def _multi_mode(self):
         """Mode of the launches that advance several steps, or None where
         steps go one by one."""
-        if not self.multi_step or self.dim != 2 or self.compute != "float32" or getattr(self, "closure", None) is not None:
+        if not self.multi_step or self.dim < 2 or self.compute != "float32" or getattr(self, "closure", None) is not None:
             return None
         if self.periodic:
             return runtime.LBM_TILE_PERIODIC
         if self._folded():
             return runtime.LBM_TILE_WALLS
-        if self._bc_batch is not None and self.batch_boundary and self._batch_entries is not None and not self._full_halo:
+        if self.dim == 2 and self._bc_batch is not None and self.batch_boundary and self._batch_entries is not None and not self._full_halo:
             return runtime.LBM_TILE_LINKS
         return None
 
@@ -904,14 +904,15 @@ class Simulation:
         mode = self._multi_mode()
         if mode is None:
             return 0
-        steps = (nsteps - 2 if mode == runtime.LBM_TILE_LINKS else nsteps) // 2 * 2
+        steps = nsteps - 2 if mode == runtime.LBM_TILE_LINKS else nsteps
         multi = self._multi_plan(mode) if steps >= 4 else None
         if multi is None:
             return 0
+        steps -= steps % multi[0].granule
         # sixteen launches to a graph once the run is long enough to repay the
         # capture (between graph nodes a launch costs 1.5 us less)
         unit = 16 * multi[0].margin
-        key = (self._F.ptr, self._Fnew.ptr, tuple(prm), mode, multi[0].shape, multi[0].margin)
+        key = (self._F.ptr, self._Fnew.ptr, tuple(prm), mode, bytes(multi[0]))
         self._multi_steps += steps
         if steps >= unit and self._graph_key != key and self._multi_steps >= 2 * unit:
             self._capture(lambda: self._enqueue_multi(mode, multi, prm, unit), key)

@@ -55,6 +55,55 @@ def test_multi_step_equals_single_steps(flow, dtype):
         sim.free()
 
 
+def _box3d(n, walls):
+    """Taylor-Green vortex or cube on n[0] x n[1] x n[2] nodes."""
+    d = W.cavity3d(n=n[0]) if walls else W.tgv3d(n=n[0])
+    dx = d["space_step"]
+    for axis, k in zip("xyz", n):
+        d["box"][axis] = [0.0, k * dx]
+    return d
+
+
+def _advection3d():
+    from demo_cases import advection_3d
+    return advection_3d(dx=1.0 / 36)
+
+
+BOXES = {
+    "tgv24": lambda: _box3d((24, 24, 24), False),
+    "tgv_flat": lambda: _box3d((9, 40, 71), False),
+    "tgv_tall": lambda: _box3d((45, 6, 33), False),
+    "cube17": lambda: _box3d((17, 17, 17), True),
+    "cube_flat": lambda: _box3d((8, 23, 70), True),
+    "cube_tall": lambda: _box3d((46, 13, 10), True),
+    "d3q6": _advection3d,
+}
+
+
+@pytest.mark.parametrize("box", list(BOXES))
+def test_two_steps_3d_equal_single_steps(box):
+    """Every split of the outermost axis the rule can take, and its choice."""
+    def make():
+        d = BOXES[box]()
+        return Simulation(d, dtype="float32", c0=None if box == "d3q6" else [1.0, 0.0, 0.0, 0.0])
+
+    single = make()
+    single.multi_step = False
+    single.run(11)
+    ref = _populations(single)
+    n0 = single.domain.shape_in[0]
+    single.free()
+    assert np.all(np.isfinite(ref))
+    splits = sorted({-(-n0 // t) for t in range(1, (n0 + 3) // 4 + 1)})
+    for planes in splits:
+        sim = make()
+        multi = sim._multi_plan(sim._multi_mode(), planes, 0)
+        assert multi is not None and multi[0].planes == planes
+        sim.run(11)
+        assert np.array_equal(_populations(sim), ref), (planes, multi[0].out[:], multi[0].tiles[:])
+        sim.free()
+
+
 def test_captured_launches_continue_the_run():
     runs = []
     for multi in (True, False):
@@ -75,6 +124,9 @@ def test_single_steps_remain_where_they_must():
     sim = Simulation(W.karman(dx=1.0 / 64), dtype="float32", c0=C0["karman"], halo="full")
     assert sim._multi_mode() is None
     sim.free()
+    sim = Simulation(W.tgv3d(n=16), dtype="float16")   # 3D in 16 bits, and small 3D grids
+    assert sim._multi_plan(sim._multi_mode()) is None
+    sim.free()
     sim = Simulation(W.tgv3d(n=16), dtype="float32")
-    assert sim._multi_mode() is None
+    assert sim._multi_plan(sim._multi_mode()) is None
     sim.free()
