@@ -195,8 +195,8 @@ def variants(args):
 # kernels, from an ncu capture of the same kernels (a property of the compiled
 # code; profiles/ncu_fp64_step_counts.md): the exact-constant D3Q19 form uses
 # 131 DADD + 14 DMUL + 84 DFMA, the printed (parity) D2Q9 form of the cavity,
-# compiled without contraction and with its walls in the step, 110 DADD + 33 DMUL
-FP64_INST_PER_NODE = {"tgv3d_256_f64": 229, "cavity_256_f64_parity": 143}
+# with its walls in the step, 69 DADD + 28 DMUL + 28 DFMA (exact rewrites)
+FP64_INST_PER_NODE = {"tgv3d_256_f64": 229, "cavity_256_f64_parity": 125}
 
 
 def fp64_roof(inst_per_node, nodes_per_s):

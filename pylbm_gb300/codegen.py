@@ -29,6 +29,7 @@ from fractions import Fraction
 import numpy as np
 import sympy as sp
 
+from .exactops import rewrite
 from .scheme import REL_U, SchemeError, to_fraction
 
 
@@ -696,7 +697,7 @@ class SchemeSource:
         out += fn("lbm_equilibrium_abs(R (&m)[LBM_Q], const R* __restrict__ prm)", ref.equilibrium("m"))
         out += fn("lbm_equilibrium_dev(R (&m)[LBM_Q], const R* __restrict__ prm)", ref.equilibrium("m"))
         out += fn("lbm_collide(R (&g)[LBM_Q], const R* __restrict__ prm)",
-                  ["R m[LBM_Q];"] + ref.moments_pull("g", "m") + ref.relaxation("m") + ref.populations("m", "g"))
+                  rewrite(ref.moments_pull("g", "m") + ref.relaxation("m") + ref.populations("m", "g"), "g")[0])
         out += self._source_half_function()
         return out
 
@@ -730,7 +731,7 @@ class SchemeSource:
                 + ("#define LBM_FLOAT_COMPUTE 1\n" if compute == "float32" else "")
                 + ("#define LBM_PLANE_STEPS 1\n" if storage == "float32" and not self.absolute_collide else "") +
                 "#include \"lbm_common.cuh\"\n"
-                "using lbm::lbm_fma;\n"
+                "using lbm::lbm_fma;\nusing lbm::lbm_neg;\n"
                 "template <typename R> __device__ __forceinline__ R lbm_sqrt(R x) { return sqrt(x); }\n"
                 "template <typename R> __device__ __forceinline__ R lbm_pow(R x, R e) { return pow(x, e); }\n"
                 + self.header() +

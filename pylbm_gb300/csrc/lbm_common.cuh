@@ -145,6 +145,15 @@ __device__ __forceinline__ F2 lbm_fma<F2>(F2 a, F2 b, F2 c) {
   return r;
 }
 
+// -a; in FP64 as a flip of the sign bit, which the FP64 pipe has no part in (a
+// negation on its own is an addition there)
+template <typename R>
+__device__ __forceinline__ R lbm_neg(R a) { return -a; }
+template <>
+__device__ __forceinline__ double lbm_neg<double>(double a) {
+  return __hiloint2double(__double2hiint(a) ^ (int)0x80000000, __double2loint(a));
+}
+
 // ---------------------------------------------------------------- geometry
 // Kernel-side copy of lbm_lattice (without the shift table).
 struct Geo {

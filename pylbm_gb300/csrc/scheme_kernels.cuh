@@ -1325,6 +1325,25 @@ inline dim3 node_grid(const lbm_lattice& l, bool with_halo) {
   return dim3(gx, gy, gz);
 }
 
+// Threads of a step block along a row of `work` nodes (or node pairs): as few
+// idle lanes as 32, 64, 96 or 128 threads allow, then the largest block.  A
+// row of 96 pairs in blocks of 128 left a quarter of the registers to warps
+// without work (D3Q19 FP16 192^3: 102 us a step).  FP64 takes 64 threads where
+// it can: its steps are bound by the FP64 pipe of the busiest SM, and
+// 256^2 nodes are 13.5 warps an SM, 14 at most in blocks of two warps against
+// 16 in blocks of four (25.8 us a step).
+inline unsigned step_block(int work) {
+  unsigned best = 0, waste = 0;
+  for (unsigned b = LBM_BLOCK; b >= 32; b -= 32) {
+    const unsigned w = ((unsigned)work + b - 1) / b * b - (unsigned)work;
+    if (best == 0 || w < waste || (w == waste && sizeof(S) == 8 && b == 64)) {
+      best = b;
+      waste = w;
+    }
+  }
+  return best;
+}
+
 // Two-node words need an even row length and every pair (z, z+1), z even, on a
 // 4-byte boundary: even element offsets of the row start, strides and planes.
 inline bool pairs_fit(const lbm_lattice& l, const void* f, const void* fnew) {
@@ -1508,18 +1527,21 @@ static int step_common(const void* f, void* fnew, const lbm_lattice* lat, const 
     return lbm::launch_check(who);
   }
   if (pairs_fit(*lat, f, fnew)) {
-    grid.x = (unsigned)((lat->n[LBM_DIM - 1] / 2 + LBM_BLOCK - 1) / LBM_BLOCK);
+    const unsigned block = step_block(lat->n[LBM_DIM - 1] / 2);
+    grid.x = ((unsigned)lat->n[LBM_DIM - 1] / 2 + block - 1) / block;
     if (periodic)
-      k_step_periodic_pairs<<<grid, LBM_BLOCK, 0, s>>>((const S*)f, (S*)fnew, a);
+      k_step_periodic_pairs<<<grid, block, 0, s>>>((const S*)f, (S*)fnew, a);
     else
-      k_step_ghost_pairs<<<grid, LBM_BLOCK, 0, s>>>((const S*)f, (S*)fnew, a);
+      k_step_ghost_pairs<<<grid, block, 0, s>>>((const S*)f, (S*)fnew, a);
     return lbm::launch_check(who);
   }
 #endif
+  const unsigned block = step_block(lat->n[LBM_DIM - 1]);
+  grid.x = ((unsigned)lat->n[LBM_DIM - 1] + block - 1) / block;
   if (periodic)
-    k_step_periodic<<<grid, LBM_BLOCK, 0, s>>>((const S*)f, (S*)fnew, a);
+    k_step_periodic<<<grid, block, 0, s>>>((const S*)f, (S*)fnew, a);
   else
-    k_step_ghost<<<grid, LBM_BLOCK, 0, s>>>((const S*)f, (S*)fnew, a);
+    k_step_ghost<<<grid, block, 0, s>>>((const S*)f, (S*)fnew, a);
   return lbm::launch_check(who);
 }
 
@@ -1555,12 +1577,15 @@ int lbm_one_time_step_walls(const void* f, void* fnew, const lbm_lattice* lat, c
   cudaStream_t s = (cudaStream_t)stream;
 #if LBM_HAS_PAIRS
   if (pairs_fit(*lat, f, fnew)) {
-    grid.x = (unsigned)((lat->n[LBM_DIM - 1] / 2 + LBM_BLOCK - 1) / LBM_BLOCK);
-    k_step_walls_pairs<<<grid, LBM_BLOCK, 0, s>>>((const S*)f, (S*)fnew, a, w);
+    const unsigned block = step_block(lat->n[LBM_DIM - 1] / 2);
+    grid.x = ((unsigned)lat->n[LBM_DIM - 1] / 2 + block - 1) / block;
+    k_step_walls_pairs<<<grid, block, 0, s>>>((const S*)f, (S*)fnew, a, w);
     return lbm::launch_check(who);
   }
 #endif
-  k_step_walls<<<grid, LBM_BLOCK, 0, s>>>((const S*)f, (S*)fnew, a, w);
+  const unsigned block = step_block(lat->n[LBM_DIM - 1]);
+  grid.x = ((unsigned)lat->n[LBM_DIM - 1] + block - 1) / block;
+  k_step_walls<<<grid, block, 0, s>>>((const S*)f, (S*)fnew, a, w);
   return lbm::launch_check(who);
 }
 

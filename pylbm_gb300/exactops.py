@@ -1,0 +1,139 @@
+"""Fewer FP64 operations with the same results: straight-line code rewritten by
+scaling and sharing only.
+
+GB300 issues FP64 at a small fraction of its FP32 rate, so the FP64 step is
+bound by the number of FP64 instructions of a node's collision.  That code is
+printed as the reference generator prints it (refforms) and has to round as
+printed, which rules out regrouping, but not these:
+
+* scaling by a power of two (and by -1) commutes with rounding, so a value is
+  carried as a scale and a base and no multiplication is spent on the scale;
+* the product of a value and a power of two is exact, so adding it is one
+  fused multiply-add that rounds like the product and the sum together;
+* with scales apart, equal prefixes of sums become equal bases and are
+  computed once (2 a + 2 b - c and -a - b + d share a + b).
+
+The results are those of the printed code, up to the sign of a zero and to
+products beyond the range of normal numbers.
+"""
+import ast
+import math
+
+
+def _power_of_two(c):
+    return c != 0.0 and math.isfinite(c) and abs(math.frexp(c)[0]) == 0.5
+
+
+class _Program:
+    def __init__(self):
+        self.lines = []
+        self.ids = {}       # operation -> base number
+        self.names = []     # base number -> C name or literal
+        self.first = {}     # mantissa -> first constant that has it
+        self.count = {"add": 0, "mul": 0, "fma": 0}
+
+    def _base(self, key, text=None, op=None):
+        """Number of the base ``key``, computed by ``text`` when it is new."""
+        if key not in self.ids:
+            self.ids[key] = len(self.names)
+            if op is None:
+                self.names.append(text)
+            else:
+                name = f"x{len(self.names)}"
+                self.lines.append(f"const R {name} = {text};")
+                self.names.append(name)
+                self.count[op] += 1
+        return self.ids[key]
+
+    def atom(self, text):
+        return (1.0, self._base(("atom", text), text))
+
+    def constant(self, c):
+        if _power_of_two(c):
+            return (c, self._base(("one",), "LBM_R(1.0)"))
+        # constants that differ by a power of two share the products of the first
+        first = self.first.setdefault(math.frexp(abs(c))[0], abs(c))
+        return (c / first, self._base(("const", first), f"LBM_R({first!r})"))
+
+    def is_one(self, b):
+        return self.ids.get(("one",)) == b
+
+    def mul(self, x, y):
+        (s, a), (t, b) = x, y
+        if self.is_one(a):
+            return (s * t, b)
+        if self.is_one(b):
+            return (s * t, a)
+        a, b = min(a, b), max(a, b)
+        return (s * t, self._base(("mul", a, b), f"{self.names[a]}*{self.names[b]}", "mul"))
+
+    def add(self, x, y):
+        if x[1] > y[1]:
+            x, y = y, x
+        (s, a), (t, b) = x, y
+        if abs(s) == abs(t):
+            r = t / s
+            return (s, self._base(("add", a, r, b), f"{self.names[a]} {'+' if r > 0 else '-'} {self.names[b]}", "add"))
+        if abs(s) != 1.0 and (abs(t) == 1.0 or abs(t) > abs(s)):  # the sum keeps a scale of one where it can
+            (s, a), (t, b) = (t, b), (s, a)
+        r = t / s
+        return (s, self._base(("add", a, r, b), f"lbm_fma<R>(LBM_R({r!r}), {self.names[b]}, {self.names[a]})", "fma"))
+
+    def value(self, v):
+        """C expression of a scaled value."""
+        s, b = v
+        if s == 1.0:
+            return self.names[b]
+        if s == -1.0:
+            return f"lbm_neg<R>({self.names[b]})"
+        if self.is_one(b):
+            return f"LBM_R({s!r})"
+        return self.names[self._base(("mul", s, b), f"LBM_R({s!r})*{self.names[b]}", "mul")]
+
+
+def rewrite(statements, result, arrays=("m", "g")):
+    """Lines of C that leave in array ``result`` what the assignments
+    ``x[i] = expression;`` leave there (``arrays`` are read and written by
+    them; other names are left as they are), and the number of additions,
+    multiplications and fused multiply-adds."""
+    p = _Program()
+    env, written = {}, []
+
+    def ev(e):
+        if isinstance(e, ast.BinOp):
+            x = ev(e.left)
+            y = ev(e.right)
+            if isinstance(e.op, ast.Add):
+                return p.add(x, y)
+            if isinstance(e.op, ast.Sub):
+                return p.add(x, (-y[0], y[1]))
+            if isinstance(e.op, ast.Mult):
+                return p.mul(x, y)
+            if isinstance(e.op, ast.Div):
+                return (1.0, p._base(("div", x, y), f"({p.value(x)})/({p.value(y)})", "mul"))
+        if isinstance(e, ast.UnaryOp) and isinstance(e.op, (ast.USub, ast.UAdd)):
+            s, b = ev(e.operand)
+            return (-s if isinstance(e.op, ast.USub) else s, b)
+        if isinstance(e, ast.Constant) and isinstance(e.value, (int, float)) and float(e.value) != 0.0:
+            return p.constant(float(e.value))
+        if isinstance(e, ast.Subscript) and isinstance(e.value, ast.Name) and e.value.id in arrays:
+            key = (e.value.id, e.slice.value)
+            if key not in env:
+                env[key] = p.atom(f"{key[0]}[{key[1]}]")
+            return env[key]
+        if isinstance(e, ast.Call):
+            args = ", ".join(p.value(ev(a)) for a in e.args)
+            name = ast.unparse(e.func)
+            return (1.0, p._base(("call", name, args), f"{name}({args})", "mul"))
+        return p.atom(ast.unparse(e))  # parameters, zero
+
+    for line in statements:
+        target, _, expr = line.strip().rstrip(";").partition("=")
+        node = ast.parse(target.strip(), mode="eval").body
+        key = (node.value.id, node.slice.value)
+        env[key] = ev(ast.parse(expr.strip(), mode="eval").body)
+        if key[0] == result and key not in written:
+            written.append(key)
+    # an array element that is read as an atom is read before it is written
+    out = [f"const R t_{a}{i} = {p.value(env[a, i])};" for a, i in written]
+    return p.lines + out + [f"{a}[{i}] = t_{a}{i};" for a, i in written], dict(p.count)
