@@ -263,24 +263,66 @@ template <> struct Pair<float> {
 
 #if defined(LBM_PAIRS) && LBM_VMAX == 1
 #define LBM_HAS_PAIRS 1
-// pulled pair of population plane `p` (already offset to node z of this row
-// and to the outer-axis neighbour), velocity component vl along the contiguous axis
-__device__ __forceinline__ lbm::F2 pull_pair(const S* __restrict__ p, int vl, int z, int nL) {
-  float lo, hi;
-  if (vl == 0) {
-    const float2 w = Pair<S>::load(p);
-    lo = w.x;
-    hi = w.y;
-  } else if (vl > 0) {  // sources z-1, z
-    const float2 w = Pair<S>::load(p);
-    hi = w.x;
-    lo = z > 0 ? Pair<S>::load(p - 2).y : Pair<S>::one(p + (nL - 1));
-  } else {  // sources z+1, z+2
-    const float2 w = Pair<S>::load(p);
-    lo = w.y;
-    hi = z + 2 < nL ? Pair<S>::load(p + 2).x : Pair<S>::one(p - z);
-  }
-  return lbm::F2(lo, hi);
+// Byte offsets of the values a pair (z, z + 1) pulls along the contiguous axis
+// -- its own word, the element below z and the one above z + 1 -- from two
+// elements before the row's first node.  The row's address and the population
+// plane's are uniform over a block, so a load costs one 32-bit register and no
+// 64-bit arithmetic per lane; a neighbour outside the word is read as one
+// element wherever it lies (next to it, in the ghost layer, or at the row's
+// other end), without branches.
+//
+// In a row of odd length the last pair holds one node: its second lane
+// computes on whatever lies there and stores nothing, and a periodic wrap
+// starts one node earlier (tail).
+struct PairAt {
+  unsigned own, below, above;
+  bool tail;  // periodic rows: z is the last node
+  bool one;   // z is the last node: store one value
+};
+__device__ __forceinline__ PairAt pair_at(int z, int below, int above) {
+  PairAt t;
+  t.tail = t.one = false;
+  t.own = (unsigned)(z + 2) * (unsigned)sizeof(S);
+  t.below = (unsigned)(below + 2) * (unsigned)sizeof(S);
+  t.above = (unsigned)(above + 2) * (unsigned)sizeof(S);
+  return t;
+}
+template <bool kOdd>
+__device__ __forceinline__ PairAt pair_at_periodic(int z, int nL) {
+  PairAt t = pair_at(z, z > 0 ? z - 1 : nL - 1, z + 2 < nL ? z + 2 : 0);
+  if (kOdd) t.tail = t.one = z + 1 == nL;
+  return t;
+}
+template <bool kOdd>
+__device__ __forceinline__ PairAt pair_at_ghost(int z, int nL) {
+  PairAt t = pair_at(z, z - 1, kOdd && z + 2 > nL ? nL : z + 2);
+  if (kOdd) t.one = z + 1 == nL;
+  return t;
+}
+
+// element offset of two elements before the first node of row (i0, i1) (halo coordinates)
+__device__ __forceinline__ long long pair_row(const Geo& g, int i0, int i1) {
+#if LBM_DIM == 1
+  return g.origin + g.h[0] - 2;
+#elif LBM_DIM == 2
+  return g.origin + (long long)i0 * g.stride[0] + g.h[1] - 2;
+#else
+  return g.origin + (long long)i0 * g.stride[0] + (long long)i1 * g.stride[1] + g.h[2] - 2;
+#endif
+}
+
+template <typename T>
+__device__ __forceinline__ T* byte_at(T* base, unsigned offset) {
+  return reinterpret_cast<T*>(reinterpret_cast<uintptr_t>(base) + offset);
+}
+
+// pulled pair of a population row, velocity component vl along the contiguous axis
+__device__ __forceinline__ lbm::F2 pull_pair(const S* __restrict__ row, int vl, const PairAt& at) {
+  const float2 w = Pair<S>::load(byte_at(row, at.own));
+  if (vl == 0) return lbm::F2(w.x, w.y);
+  if (vl > 0) return lbm::F2(Pair<S>::one(byte_at(row, at.below)), w.x);
+  const float up = Pair<S>::one(byte_at(row, at.above));
+  return lbm::F2(at.tail ? up : w.y, up);
 }
 
 // the velocity component along the last axis and the outer offset of population k
@@ -296,35 +338,41 @@ __device__ __forceinline__ lbm::F2 pull_pair(const S* __restrict__ p, int vl, in
 #endif
 
 // the pulled values of the two nodes (z, z + 1) of a row, periodic wrap
-__device__ __forceinline__ void pull_pairs(const S* __restrict__ f, const Geo& g, int i0, int i1, int i2, int z,
-                                           int nL, lbm::F2 (&gv)[LBM_Q]) {
-  const long long o = lbm::node_offset(g, i0, i1, i2);
+__device__ __forceinline__ void pull_pairs(const S* __restrict__ f, const Geo& g, int i0, int i1, const PairAt& at,
+                                           lbm::F2 (&gv)[LBM_Q]) {
+  const S* row = f + pair_row(g, i0, i1);
   long long off0[3] = {0, 0, 0}, off1[3] = {0, 0, 0};
 #pragma unroll
   for (int s = -1; s <= 1; ++s) {
     if (LBM_DIM > 1) off0[s + 1] = wrap_off(i0, s, g.n[0], g.h[0], g.stride[0]);
     if (LBM_DIM > 2) off1[s + 1] = wrap_off(i1, s, g.n[1], g.h[1], g.stride[1]);
   }
+  (void)off0;
   (void)off1;
 #define LBM_PULL_PAIR(k, vx, vy, vz) \
-  gv[k] = pull_pair(f + o + (long long)(k) * g.vstride + LBM_OUTER(vx, vy, vz), LBM_VL(vx, vy, vz), z, nL);
+  gv[k] = pull_pair(row + ((long long)(k) * g.vstride + LBM_OUTER(vx, vy, vz)), LBM_VL(vx, vy, vz), at);
   LBM_FOR_EACH_V(LBM_PULL_PAIR)
 #undef LBM_PULL_PAIR
 }
 
 __device__ __forceinline__ void collide_store_pairs(S* __restrict__ fnew, const Geo& g, const lbm::F2 (&prm)[kPrm],
-                                                    int i0, int i1, int i2, lbm::F2 (&gv)[LBM_Q]) {
-  const long long o = lbm::node_offset(g, i0, i1, i2);
+                                                    int i0, int i1, const PairAt& at, lbm::F2 (&gv)[LBM_Q]) {
+  S* row = fnew + pair_row(g, i0, i1);
   lbm_collide<lbm::F2>(gv, prm);
+  if (at.one) {
 #pragma unroll
-  for (int k = 0; k < LBM_Q; ++k) Pair<S>::store(fnew + o + (long long)k * g.vstride, gv[k].v);
+    for (int k = 0; k < LBM_Q; ++k) Store<S>::store(byte_at(row + (long long)k * g.vstride, at.own), gv[k].v.x);
+    return;
+  }
+#pragma unroll
+  for (int k = 0; k < LBM_Q; ++k) Pair<S>::store(byte_at(row + (long long)k * g.vstride, at.own), gv[k].v);
 }
 
 __device__ __forceinline__ void step_pair(const S* __restrict__ f, S* __restrict__ fnew, const Geo& g,
-                                          const lbm::F2 (&prm)[kPrm], int i0, int i1, int i2, int z, int nL) {
+                                          const lbm::F2 (&prm)[kPrm], int i0, int i1, const PairAt& at) {
   lbm::F2 gv[LBM_Q];
-  pull_pairs(f, g, i0, i1, i2, z, nL, gv);
-  collide_store_pairs(fnew, g, prm, i0, i1, i2, gv);
+  pull_pairs(f, g, i0, i1, at, gv);
+  collide_store_pairs(fnew, g, prm, i0, i1, at, gv);
 }
 
 // eight resident blocks of LBM_BLOCK threads per SM: 64 registers, no spills
@@ -334,19 +382,6 @@ __device__ __forceinline__ void step_pair(const S* __restrict__ f, S* __restrict
 #define LBM_PAIRS_MIN_BLOCKS 8
 #endif
 
-// Bounded domains: the pull reads the ghost layer (refreshed and written by
-// the boundary methods before the step), so the two sources of a pair need
-// no wrap.  For z = 0 the word at p - 2 holds (z - 2, z - 1): z - 1 is the
-// ghost, z - 2 the last element of the row before (in the buffer: every
-// interior row follows a ghost plane).  For the last pair the word at p + 2
-// holds (n, n + 1): n is the ghost, n + 1 lies in the row after.
-__device__ __forceinline__ lbm::F2 pull_pair_ghost(const S* __restrict__ p, int vl) {
-  const float2 w = Pair<S>::load(p);
-  if (vl == 0) return lbm::F2(w.x, w.y);
-  if (vl > 0) return lbm::F2(Pair<S>::load(p - 2).y, w.x);
-  return lbm::F2(w.y, Pair<S>::load(p + 2).x);
-}
-
 #if LBM_DIM == 1
 #define LBM_OUTER_GHOST(vx, vy, vz) 0LL
 #elif LBM_DIM == 2
@@ -355,38 +390,35 @@ __device__ __forceinline__ lbm::F2 pull_pair_ghost(const S* __restrict__ p, int 
 #define LBM_OUTER_GHOST(vx, vy, vz) (-((long long)(vx) * a.g.stride[0] + (long long)(vy) * a.g.stride[1]))
 #endif
 
+template <bool kOdd>
 __global__ void __launch_bounds__(LBM_BLOCK, LBM_PAIRS_MIN_BLOCKS) k_step_ghost_pairs(const S* __restrict__ f,
                                                                                     S* __restrict__ fnew,
                                                                                     StepArgs a) {
   const int z = 2 * (blockIdx.x * blockDim.x + threadIdx.x);
   const int nL = a.g.n[LBM_DIM - 1];
   if (z >= nL) return;
-  int i0, i1, i2;
 #if LBM_DIM == 1
-  i0 = z + a.g.h[0];
-  i1 = i2 = 0;
+  const int i0 = 0, i1 = 0;
 #elif LBM_DIM == 2
-  i0 = blockIdx.y + a.g.h[0];
-  i1 = z + a.g.h[1];
-  i2 = 0;
+  const int i0 = blockIdx.y + a.g.h[0], i1 = 0;
 #else
-  i0 = blockIdx.z + a.g.h[0];
-  i1 = blockIdx.y + a.g.h[1];
-  i2 = z + a.g.h[2];
+  const int i0 = blockIdx.z + a.g.h[0], i1 = blockIdx.y + a.g.h[1];
 #endif
   lbm::F2 prm[kPrm];
 #pragma unroll
   for (int p = 0; p < kPrm; ++p) prm[p] = lbm::F2((float)a.prm[p]);
-  const long long o = lbm::node_offset(a.g, i0, i1, i2);
+  const S* row = f + pair_row(a.g, i0, i1);
+  const PairAt at = pair_at_ghost<kOdd>(z, nL);
   lbm::F2 gv[LBM_Q];
 #define LBM_PULL_GHOST(k, vx, vy, vz) \
-  gv[k] = pull_pair_ghost(f + o + (long long)(k) * a.g.vstride + LBM_OUTER_GHOST(vx, vy, vz), LBM_VL(vx, vy, vz));
+  gv[k] = pull_pair(row + ((long long)(k) * a.g.vstride + LBM_OUTER_GHOST(vx, vy, vz)), LBM_VL(vx, vy, vz), at);
   LBM_FOR_EACH_V(LBM_PULL_GHOST)
 #undef LBM_PULL_GHOST
-  collide_store_pairs(fnew, a.g, prm, i0, i1, i2, gv);
+  collide_store_pairs(fnew, a.g, prm, i0, i1, at, gv);
 }
 
 // the box-wall fold for two nodes (z, z + 1) per thread (16-bit storage)
+template <bool kOdd>
 __global__ void __launch_bounds__(LBM_BLOCK, LBM_PAIRS_MIN_BLOCKS) k_step_walls_pairs(const S* __restrict__ f,
                                                                                      S* __restrict__ fnew,
                                                                                      StepArgs a, WallArgs w) {
@@ -394,27 +426,23 @@ __global__ void __launch_bounds__(LBM_BLOCK, LBM_PAIRS_MIN_BLOCKS) k_step_walls_
   const int z = 2 * (blockIdx.x * blockDim.x + threadIdx.x);
   const int nL = a.g.n[L];
   if (z >= nL) return;
-  int i0, i1, i2;
 #if LBM_DIM == 1
-  i0 = z + a.g.h[0];
-  i1 = i2 = 0;
+  const int i0 = 0, i1 = 0;
 #elif LBM_DIM == 2
-  i0 = blockIdx.y + a.g.h[0];
-  i1 = z + a.g.h[1];
-  i2 = 0;
+  const int i0 = blockIdx.y + a.g.h[0], i1 = 0;
 #else
-  i0 = blockIdx.z + a.g.h[0];
-  i1 = blockIdx.y + a.g.h[1];
-  i2 = z + a.g.h[2];
+  const int i0 = blockIdx.z + a.g.h[0], i1 = blockIdx.y + a.g.h[1];
 #endif
   lbm::F2 prm[kPrm];
 #pragma unroll
   for (int p = 0; p < kPrm; ++p) prm[p] = lbm::F2((float)a.prm[p]);
-  const long long o = lbm::node_offset(a.g, i0, i1, i2);
+  const S* row = f + pair_row(a.g, i0, i1);
+  const PairAt at = pair_at_ghost<kOdd>(z, nL);
   // faces of the outer axes (shared by both nodes) and of the contiguous axis (per node)
   const bool lo0 = LBM_DIM > 1 && i0 == a.g.h[0], hi0 = LBM_DIM > 1 && i0 == a.g.h[0] + a.g.n[0] - 1;
   const bool lo1 = LBM_DIM > 2 && i1 == a.g.h[1], hi1 = LBM_DIM > 2 && i1 == a.g.h[1] + a.g.n[1] - 1;
-  const bool first = z == 0, last = z + 2 == nL;
+  // the wall above the row: the second node's, or the only one's
+  const bool first = z == 0, last = z + 2 == nL, only = kOdd && z + 1 == nL;
   lbm::F2 gv[LBM_Q];
   // wall signature 9 (o0+1) + 3 (o1+1) + (o2+1): the outer axes' part, and the
   // weight of the contiguous axis
@@ -432,11 +460,11 @@ __global__ void __launch_bounds__(LBM_BLOCK, LBM_PAIRS_MIN_BLOCKS) k_step_walls_
   {                                                                                                   \
     const int vl = LBM_VL(vx, vy, vz);                                                                \
     const int base = LBM_WALL_BASE(vx, vy, vz);                                                       \
-    const int s0 = base + wL * wall_off(vl, first, false);                                            \
+    const int s0 = base + wL * wall_off(vl, first, only);                                             \
     const int s1 = base + wL * wall_off(vl, false, last);                                             \
-    gv[k] = pull_pair_ghost(f + o + (long long)(k) * a.g.vstride + LBM_OUTER_GHOST(vx, vy, vz), vl); \
+    gv[k] = pull_pair(row + ((long long)(k) * a.g.vstride + LBM_OUTER_GHOST(vx, vy, vz)), vl, at);     \
     if (s0 != 13 || s1 != 13) {                                                                       \
-      const float2 bb = Pair<S>::load(f + o + (long long)w.sym[k] * a.g.vstride);                     \
+      const float2 bb = Pair<S>::load(byte_at(row + (long long)w.sym[k] * a.g.vstride, at.own));                     \
       if (s0 != 13) gv[k].v.x = through_storage(bb.x + w.c[k][s0]);                                 \
       if (s1 != 13) gv[k].v.y = through_storage(bb.y + w.c[k][s1]);                                 \
     }                                                                                                 \
@@ -447,16 +475,17 @@ __global__ void __launch_bounds__(LBM_BLOCK, LBM_PAIRS_MIN_BLOCKS) k_step_walls_
     // source is the wall normal to the contiguous axis is replaced, so only
     // that thread's few loads diverge
 #define LBM_PULL_GHOST_W(k, vx, vy, vz) \
-  gv[k] = pull_pair_ghost(f + o + (long long)(k) * a.g.vstride + LBM_OUTER_GHOST(vx, vy, vz), LBM_VL(vx, vy, vz));
+  gv[k] = pull_pair(row + ((long long)(k) * a.g.vstride + LBM_OUTER_GHOST(vx, vy, vz)), LBM_VL(vx, vy, vz), at);
     LBM_FOR_EACH_V(LBM_PULL_GHOST_W)
 #undef LBM_PULL_GHOST_W
-    if (first || last) {
+    if (first || last || only) {
 #define LBM_FIX_END_PAIR(k, vx, vy, vz)                                                       \
   {                                                                                           \
     const int vl = LBM_VL(vx, vy, vz);                                                        \
-    if ((first && vl > 0) || (last && vl < 0)) {                                             \
-      const float2 bb = Pair<S>::load(f + o + (long long)w.sym[k] * a.g.vstride);             \
+    if ((first && vl > 0) || ((last || only) && vl < 0)) {                                    \
+      const float2 bb = Pair<S>::load(byte_at(row + (long long)w.sym[k] * a.g.vstride, at.own));             \
       if (first && vl > 0) gv[k].v.x = through_storage(bb.x + w.c[k][13 - wL]);               \
+      if (only && vl < 0) gv[k].v.x = through_storage(bb.x + w.c[k][13 + wL]);                \
       if (last && vl < 0) gv[k].v.y = through_storage(bb.y + w.c[k][13 + wL]);                \
     }                                                                                         \
   }
@@ -468,35 +497,30 @@ __global__ void __launch_bounds__(LBM_BLOCK, LBM_PAIRS_MIN_BLOCKS) k_step_walls_
   }
 #undef LBM_PULL_WALL_PAIR
 #undef LBM_WALL_BASE
-  collide_store_pairs(fnew, a.g, prm, i0, i1, i2, gv);
+  collide_store_pairs(fnew, a.g, prm, i0, i1, at, gv);
 }
 
 #ifndef LBM_ENSEMBLE_ROW_PAIRS
 #define LBM_ENSEMBLE_ROW_PAIRS 1
 #endif
+template <bool kOdd>
 __global__ void __launch_bounds__(LBM_BLOCK, LBM_PAIRS_MIN_BLOCKS) k_step_periodic_pairs(const S* __restrict__ f, S* __restrict__ fnew,
                                                                    StepArgs a) {
   constexpr int L = LBM_DIM - 1;
   const int z = 2 * (blockIdx.x * blockDim.x + threadIdx.x);
   const int nL = a.g.n[L];
   if (z >= nL) return;
-  int i0, i1, i2;
 #if LBM_DIM == 1
-  i0 = z + a.g.h[0];
-  i1 = i2 = 0;
+  const int i0 = 0, i1 = 0;
 #elif LBM_DIM == 2
-  i0 = blockIdx.y + a.g.h[0];
-  i1 = z + a.g.h[1];
-  i2 = 0;
+  const int i0 = blockIdx.y + a.g.h[0], i1 = 0;
 #else
-  i0 = blockIdx.z + a.g.h[0];
-  i1 = blockIdx.y + a.g.h[1];
-  i2 = z + a.g.h[2];
+  const int i0 = blockIdx.z + a.g.h[0], i1 = blockIdx.y + a.g.h[1];
 #endif
   lbm::F2 prm[kPrm];
 #pragma unroll
   for (int p = 0; p < kPrm; ++p) prm[p] = lbm::F2((float)a.prm[p]);
-  step_pair(f, fnew, a.g, prm, i0, i1, i2, z, nL);
+  step_pair(f, fnew, a.g, prm, i0, i1, pair_at_periodic<kOdd>(z, nL));
 }
 
 // ---------------------------------------------------------------------------
@@ -617,11 +641,7 @@ __global__ void __launch_bounds__(kStagedThreads) k_step_periodic_staged(const S
 #define LBM_PULL_STAGED(k, vx, vy, vz) gv[k] = staged_pair(stage + (size_t)(k) * nL, LBM_VL(vx, vy, vz), z, nL);
       LBM_FOR_EACH_V(LBM_PULL_STAGED)
 #undef LBM_PULL_STAGED
-#if LBM_DIM == 3
-      collide_store_pairs(fnew, g, prm, x0 + g.h[0], x1 + g.h[1], z + g.h[2], gv);
-#else
-      collide_store_pairs(fnew, g, prm, x0 + g.h[0], z + g.h[1], 0, gv);
-#endif
+      collide_store_pairs(fnew, g, prm, x0 + g.h[0], x1 + g.h[1], pair_at_ghost<false>(z, nL), gv);
     }
     __syncwarp();
     if (lane == 0) lbm::mbar_arrive(&empty[s]);
@@ -678,7 +698,7 @@ __device__ __forceinline__ void step_node(const S* __restrict__ f, S* __restrict
 // kPairsOnly: every instance carries LBM_INSTANCE_PAIRS (the caller checks),
 // so the kernel holds the two-node path alone (fewer registers).
 template <bool kPairsOnly>
-__global__ void __launch_bounds__(LBM_ENSEMBLE_MAX_BLOCK) k_step_ensemble(S* __restrict__ arena,
+__global__ void __launch_bounds__(LBM_ENSEMBLE_MAX_BLOCK, !LBM_HAS_PAIRS ? 0 : LBM_Q <= 9 ? 4 : 2) k_step_ensemble(S* __restrict__ arena,
                                                                           const lbm_instance* __restrict__ inst,
                                                                           const int* __restrict__ tile_inst,
                                                                           int ntiles, int rows_per_tile, int parity) {
@@ -716,6 +736,7 @@ __global__ void __launch_bounds__(LBM_ENSEMBLE_MAX_BLOCK) k_step_ensemble(S* __r
       lbm::F2 prm2[kPrm];
 #pragma unroll
       for (int p = 0; p < kPrm; ++p) prm2[p] = lbm::F2((float)I->prm[p < LBM_MAX_PRM ? p : 0]);
+      const PairAt at = pair_at_periodic<false>(z, nL);
       int r = r0;
 #if LBM_ENSEMBLE_ROW_PAIRS
       // two rows at a time: both rows' loads are issued before either collide
@@ -724,16 +745,16 @@ __global__ void __launch_bounds__(LBM_ENSEMBLE_MAX_BLOCK) k_step_ensemble(S* __r
         row_coords(g, r, z, a);
         row_coords(g, r + 1, z, b);
         lbm::F2 ga[LBM_Q], gb[LBM_Q];
-        pull_pairs(f, g, a[0], a[1], a[2], z, nL, ga);
-        pull_pairs(f, g, b[0], b[1], b[2], z, nL, gb);
-        collide_store_pairs(fnew, g, prm2, a[0], a[1], a[2], ga);
-        collide_store_pairs(fnew, g, prm2, b[0], b[1], b[2], gb);
+        pull_pairs(f, g, a[0], a[1], at, ga);
+        pull_pairs(f, g, b[0], b[1], at, gb);
+        collide_store_pairs(fnew, g, prm2, a[0], a[1], at, ga);
+        collide_store_pairs(fnew, g, prm2, b[0], b[1], at, gb);
       }
 #endif
       for (; r < r1; ++r) {
         int idx[3];
         row_coords(g, r, z, idx);
-        step_pair(f, fnew, g, prm2, idx[0], idx[1], idx[2], z, nL);
+        step_pair(f, fnew, g, prm2, idx[0], idx[1], at);
       }
       continue;
     }
@@ -1344,11 +1365,13 @@ inline unsigned step_block(int work) {
   return best;
 }
 
-// Two-node words need an even row length and every pair (z, z+1), z even, on a
-// 4-byte boundary: even element offsets of the row start, strides and planes.
+// Two-node words need every pair (z, z+1), z even, on a 4-byte boundary: even
+// element offsets of the row start, strides and planes.  A row of odd length
+// ends in a pair of one node (its word reaches one element beyond the row,
+// into the ghost layer).
 inline bool pairs_fit(const lbm_lattice& l, const void* f, const void* fnew) {
   const int L = LBM_DIM - 1;
-  if (l.n[L] % 2 || (l.origin + l.halo[L]) % 2 || l.vstride % 2) return false;
+  if (l.halo[L] < 1 || (l.origin + l.halo[L]) % 2 || l.vstride % 2) return false;
   for (int d = 0; d < L; ++d)
     if (l.stride[d] % 2) return false;
   return ((uintptr_t)f % 4 == 0) && ((uintptr_t)fnew % 4 == 0);
@@ -1358,7 +1381,7 @@ inline bool pairs_fit(const lbm_lattice& l, const void* f, const void* fnew) {
 // the staged step applies: 2D or 3D rows whose bytes and starts suit bulk copies
 inline bool staged_fits(const lbm_lattice& l, const void* f, const void* fnew) {
   const int L = LBM_DIM - 1;
-  if (LBM_DIM < 2 || !pairs_fit(l, f, fnew)) return false;
+  if (LBM_DIM < 2 || l.n[L] % 2 || !pairs_fit(l, f, fnew)) return false;
   const long long es = (long long)sizeof(S);
   if ((l.n[L] * es) % 16 || l.n[L] > 1024) return false;  // row bytes: multiple of 16, stage within shared memory
   if (((l.origin + l.halo[L]) * es) % 16 || (l.vstride * es) % 16) return false;
@@ -1527,12 +1550,17 @@ static int step_common(const void* f, void* fnew, const lbm_lattice* lat, const 
     return lbm::launch_check(who);
   }
   if (pairs_fit(*lat, f, fnew)) {
-    const unsigned block = step_block(lat->n[LBM_DIM - 1] / 2);
-    grid.x = ((unsigned)lat->n[LBM_DIM - 1] / 2 + block - 1) / block;
-    if (periodic)
-      k_step_periodic_pairs<<<grid, block, 0, s>>>((const S*)f, (S*)fnew, a);
+    const unsigned pairs = ((unsigned)lat->n[LBM_DIM - 1] + 1) / 2, block = step_block((int)pairs);
+    grid.x = (pairs + block - 1) / block;
+    const bool odd = lat->n[LBM_DIM - 1] % 2;
+    if (periodic && odd)
+      k_step_periodic_pairs<true><<<grid, block, 0, s>>>((const S*)f, (S*)fnew, a);
+    else if (periodic)
+      k_step_periodic_pairs<false><<<grid, block, 0, s>>>((const S*)f, (S*)fnew, a);
+    else if (odd)
+      k_step_ghost_pairs<true><<<grid, block, 0, s>>>((const S*)f, (S*)fnew, a);
     else
-      k_step_ghost_pairs<<<grid, block, 0, s>>>((const S*)f, (S*)fnew, a);
+      k_step_ghost_pairs<false><<<grid, block, 0, s>>>((const S*)f, (S*)fnew, a);
     return lbm::launch_check(who);
   }
 #endif
@@ -1577,9 +1605,12 @@ int lbm_one_time_step_walls(const void* f, void* fnew, const lbm_lattice* lat, c
   cudaStream_t s = (cudaStream_t)stream;
 #if LBM_HAS_PAIRS
   if (pairs_fit(*lat, f, fnew)) {
-    const unsigned block = step_block(lat->n[LBM_DIM - 1] / 2);
-    grid.x = ((unsigned)lat->n[LBM_DIM - 1] / 2 + block - 1) / block;
-    k_step_walls_pairs<<<grid, block, 0, s>>>((const S*)f, (S*)fnew, a, w);
+    const unsigned pairs = ((unsigned)lat->n[LBM_DIM - 1] + 1) / 2, block = step_block((int)pairs);
+    grid.x = (pairs + block - 1) / block;
+    if (lat->n[LBM_DIM - 1] % 2)
+      k_step_walls_pairs<true><<<grid, block, 0, s>>>((const S*)f, (S*)fnew, a, w);
+    else
+      k_step_walls_pairs<false><<<grid, block, 0, s>>>((const S*)f, (S*)fnew, a, w);
     return lbm::launch_check(who);
   }
 #endif
