@@ -232,10 +232,9 @@ class Simulation:
         self._walls = None          # (constants nv x 27, opposite populations) of lbm_one_time_step_walls
         self.multi_step = True      # run() advances several steps per launch where the lattice allows it
         self._multi = {}            # (lbm_tile_plan, lbm_tile_boundary) by mode
-        self._multi_steps = 0       # steps advanced that way
         self._batch_entries = None  # links of the batched boundary launch, FP32 form, for the tiles
-        self._graph = None
-        self._graph_key = None
+        self._graphs = {}           # captured steps by what they launch
+        self._graph_steps = 0       # steps run since the graphs were dropped
         self._need_init = True
         if initialize:
             self._initialize()
@@ -847,10 +846,10 @@ class Simulation:
         self._m_partial = False
 
     def _drop_graph(self):
-        if self._graph is not None:
-            self._core.lbm_graph_destroy(self._graph)
-        self._graph = None
-        self._graph_key = None
+        for graph in self._graphs.values():
+            self._core.lbm_graph_destroy(graph)
+        self._graphs = {}
+        self._graph_steps = 0
 
     def _multi_mode(self):
         """Mode of the launches that advance several steps, or None where
@@ -909,18 +908,8 @@ class Simulation:
         if multi is None:
             return 0
         steps -= steps % multi[0].granule
-        # sixteen launches to a graph once the run is long enough to repay the
-        # capture (between graph nodes a launch costs 1.5 us less)
-        unit = 16 * multi[0].margin
-        key = (self._F.ptr, self._Fnew.ptr, tuple(prm), mode, bytes(multi[0]))
-        self._multi_steps += steps
-        if steps >= unit and self._graph_key != key and self._multi_steps >= 2 * unit:
-            self._capture(lambda: self._enqueue_multi(mode, multi, prm, unit), key)
-        done = 0
-        if self._graph_key == key:
-            for _ in range(steps // unit):
-                runtime.check(self._core.lbm_graph_launch(self._graph, self._stream))
-            done = steps // unit * unit
+        done = self._replay(steps, 16 * multi[0].margin, ("multi", mode, bytes(multi[0])), prm,
+                            lambda unit: self._enqueue_multi(mode, multi, prm, unit))
         if steps > done:
             self._enqueue_multi(mode, multi, prm, steps - done)
         return steps
@@ -931,13 +920,36 @@ class Simulation:
             self._F.handle, self._Fnew.handle, ctypes.byref(self._lat), prm.ctypes.data_as(ctypes.c_void_p),
             ctypes.byref(plan), steps, mode, ctypes.byref(bnd), self._stream))
 
-    def _enqueue_two_steps(self, prm):
-        self._enqueue_step(self._F, self._Fnew, prm)
-        self._enqueue_step(self._Fnew, self._F, prm)
+    def _enqueue_steps(self, prm, steps):
+        """An even number of steps, one launch sequence each, from F back to F."""
+        for _ in range(steps // 2):
+            self._enqueue_step(self._F, self._Fnew, prm)
+            self._enqueue_step(self._Fnew, self._F, prm)
 
-    def _capture(self, enqueue, key):
-        """Capture steps that leave the populations in F into one executable graph."""
-        self._drop_graph()
+    def _replay(self, steps, unit, kind, prm, enqueue, always=False):
+        """Advance up to ``steps`` steps by replays of a graph of ``unit`` steps
+        (``enqueue(unit)``, which leaves the populations in F); returns their
+        number.  A graph of sixteen launches or more is captured once the steps
+        so far repay the capture: between graphs the GPU loses about 1.5 us more
+        than between launches of one graph, and a graph of two short steps waits
+        for a whole multiple of 2 us."""
+        key = (kind, unit, self._F.ptr, self._Fnew.ptr, tuple(prm))
+        if steps < unit:
+            return 0
+        graph = self._graphs.get(key)
+        if graph is None:
+            self._graph_steps += steps
+            if not always and self._graph_steps < 2 * unit:
+                return 0
+            if len(self._graphs) >= 4:
+                self._drop_graph()
+            graph = self._graphs[key] = self._capture(lambda: enqueue(unit))
+        for _ in range(steps // unit):
+            runtime.check(self._core.lbm_graph_launch(graph, self._stream))
+        return steps // unit * unit
+
+    def _capture(self, enqueue):
+        """The work that ``enqueue`` puts on the stream as an executable graph."""
         runtime.check(self._core.lbm_graph_begin(self._stream))
         try:
             enqueue()
@@ -945,8 +957,7 @@ class Simulation:
             g = ctypes.c_void_p()
             rc = self._core.lbm_graph_end(self._stream, ctypes.byref(g))
         runtime.check(rc)
-        self._graph = g
-        self._graph_key = key
+        return g
 
     def run(self, nsteps, graph=True):
         """Advance ``nsteps`` time steps (same result as calling one_time_step)."""
@@ -959,23 +970,19 @@ class Simulation:
                 self.one_time_step()
             return
         prm = self._prm()
-        many = self._run_multi(nsteps, prm)
-        pairs = 0
-        if not many:
-            key = (self._F.ptr, self._Fnew.ptr, tuple(prm), self._folded(), self.batch_boundary,
-                   getattr(self, "closure_kernel", None))
-            if self._graph_key != key:
-                self._capture(lambda: self._enqueue_two_steps(prm), key)
-            pairs = nsteps // 2
-        for _ in range(pairs):
-            runtime.check(self._core.lbm_graph_launch(self._graph, self._stream))
-        for _ in range(many + 2 * pairs):
+        done = self._run_multi(nsteps, prm)
+        if not done:
+            kind = ("single", self._folded(), self.batch_boundary, getattr(self, "closure_kernel", None))
+            steps = nsteps // 2 * 2
+            for unit in (16, 2):
+                done += self._replay(steps - done, unit, kind, prm, lambda n: self._enqueue_steps(prm, n), unit == 2)
+        for _ in range(done):
             self.t += self.dt
-        self.nt += many + 2 * pairs
+        self.nt += done
         self._update_m = True
         self._eq_pending = False
         self._m_cache = {}
-        for _ in range(nsteps - many - 2 * pairs):
+        for _ in range(nsteps - done):
             self.one_time_step()
 
     def synchronize(self):

@@ -117,6 +117,24 @@ def test_captured_launches_continue_the_run():
     assert np.array_equal(*runs)
 
 
+@pytest.mark.parametrize("flow", ["cavity33", "karman"])
+def test_captured_single_steps_equal_calls(flow):
+    """Runs long enough for the graph of sixteen steps, its remainder and an odd step."""
+    runs = []
+    for captured in (True, False):
+        sim = Simulation(FLOWS[flow]())
+        for steps in (37, 35, 5):
+            if captured:
+                sim.run(steps)
+            else:
+                for _ in range(steps):
+                    sim.one_time_step()
+        assert sim.nt == 77
+        runs.append((_populations(sim), sim.t))
+        sim.free()
+    assert np.array_equal(runs[0][0], runs[1][0]) and runs[0][1] == runs[1][1]
+
+
 def test_single_steps_remain_where_they_must():
     sim = Simulation(W.cavity(n=32))   # FP64
     assert sim._multi_mode() is None
