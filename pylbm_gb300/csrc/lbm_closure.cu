@@ -325,8 +325,10 @@ struct AdamArgs {
   int n;
 };
 
+// Adam, and the updated weight's BF16 copies at their places in both layouts
+// (what k_mlp_sync writes, without a launch of its own)
 __global__ void k_mlp_adam(float* __restrict__ p, float* __restrict__ m, float* __restrict__ v,
-                           float* __restrict__ grad, AdamArgs a) {
+                           float* __restrict__ grad, __nv_bfloat16* __restrict__ wb, AdamArgs a) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= a.n) return;
   const float gr = grad[i];
@@ -334,8 +336,22 @@ __global__ void k_mlp_adam(float* __restrict__ p, float* __restrict__ m, float* 
   const float vv = a.beta2 * v[i] + (1.0f - a.beta2) * gr * gr;
   m[i] = mm;
   v[i] = vv;
-  p[i] -= a.lr * (mm / a.bc1) / (sqrtf(vv / a.bc2) + a.eps);
+  const float w = p[i] - a.lr * (mm / a.bc1) / (sqrtf(vv / a.bc2) + a.eps);
+  p[i] = w;
   grad[i] = 0.0f;
+  const __nv_bfloat16 b = __float2bfloat16_rn(w);
+  if (i < PB1) {
+    wb[BW1T + frag_index((i - PW1) / IN, (i - PW1) % IN, IN)] = b;
+  } else if (i >= PW2 && i < PB2) {
+    const int out = (i - PW2) / H, in = (i - PW2) % H;
+    wb[BW2T + frag_index(out, in, H)] = b;
+    wb[BW2N + frag_index(in, out, H)] = b;
+  } else if (i >= PW3 && i < PB3) {
+    const int out = (i - PW3) / H, in = (i - PW3) % H;
+    wb[BW3T + frag_index(out, in, H)] = b;
+    wb[BW3N + frag_index(in, out, 16)] = b;
+    wb[BW3N + frag_index(in, out + OUT, 16)] = __float2bfloat16(0.0f);
+  }
 }
 
 __global__ void __launch_bounds__(32 * kWarps) k_mlp_infer(const __nv_bfloat16* __restrict__ x, int n,
@@ -494,10 +510,8 @@ int lbm_mlp_adam(float* params, float* m, float* v, float* grad, float lr, float
   a.bc2 = 1.0f - powf(beta2, (float)step);
   a.n = NPARAM;
   cudaStream_t st = (cudaStream_t)stream;
-  k_mlp_adam<<<(NPARAM + 255) / 256, 256, 0, st>>>(params, m, v, grad, a);
-  int rc = launch_check("lbm_mlp_adam");
-  if (rc) return rc;
-  return lbm_mlp_sync_weights(params, wbf16, stream);
+  k_mlp_adam<<<(NPARAM + 127) / 128, 128, 0, st>>>(params, m, v, grad, (__nv_bfloat16*)wbf16, a);
+  return launch_check("lbm_mlp_adam");
 }
 
 }  // extern "C"

@@ -98,6 +98,13 @@ __device__ __forceinline__ void frag_source(int idx, int K, int& n, int& k) {
   k = kt * 16 + 2 * t + (j & 1) + ((j & 2) ? 8 : 0);
 }
 
+// position of element (n, k) of an [N][K] matrix in fragment order
+__device__ __forceinline__ int frag_index(int n, int k, int K) {
+  const int tile = (n >> 3) * (K / 16) + (k >> 4);
+  const int lane = (n & 7) * 4 + ((k & 7) >> 1);
+  return tile * 128 + lane * 4 + (k & 1) + ((k & 8) ? 2 : 0);
+}
+
 __device__ __forceinline__ void load_b(const __nv_bfloat16* w, int K, int nt, int kt, int lane, uint32_t& b0,
                                        uint32_t& b1) {
   const uint2 v = reinterpret_cast<const uint2*>(w)[(nt * (K / 16) + kt) * 32 + lane];

@@ -225,6 +225,19 @@ __device__ __forceinline__ void backward_epilogue(uint32_t t_acc, uint32_t t_z, 
   }
 }
 
+// four consecutive floats added in global memory, in one operation where p is
+// 16-byte aligned: every block adds all 5768 gradients, and the L2's atomic
+// operations bound that part
+__device__ __forceinline__ void add4(float* p, const float* v, bool wide) {
+  if (wide) {
+    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3])
+                 : "memory");
+    return;
+  }
+#pragma unroll
+  for (int j = 0; j < 4; ++j) atomicAdd(p + j, v[j]);
+}
+
 __global__ void __launch_bounds__(kThreads, 1) k_mlp_train_tc(const __nv_bfloat16* __restrict__ x,
                                                               const float* __restrict__ target, int n,
                                                               const float* __restrict__ params,
@@ -245,13 +258,24 @@ __global__ void __launch_bounds__(kThreads, 1) k_mlp_train_tc(const __nv_bfloat1
   stage_bf16(smem + kW1, params + PW1, H, H, IN, tid, kThreads);
   stage_bf16(smem + kW2, params + PW2, H, H, H, tid, kThreads);
   stage_bf16(smem + kW3, params + PW3, kN3, OUT, H, tid, kThreads);
-  for (int e = tid; e < H * 16; e += kThreads) {
-    const int i = e >> 4, o = e & 15;
-    store_bf16(smem + kW3T, core_offset(i, o, 16), o < OUT ? params[PW3 + o * H + i] : 0.0f);
+  // the transposed ones by columns: lanes read consecutive inputs i of eight
+  // outputs and store one row's eight values (element by element, each lane in
+  // a row of its own, staging and the gradients' additions took 23 us of a
+  // 35 us launch at 32768 samples; now 18.6 us in all)
+  for (int e = tid; e < H * 2; e += kThreads) {
+    const int i = e % H, o = e / H * 8;
+    float v[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = o + j < OUT ? params[PW3 + (o + j) * H + i] : 0.0f;
+    store8_bf16(smem + kW3T, core_offset(i, o, 16), v);
   }
-  for (int e = tid; e < H * H; e += kThreads) {
-    const int i = e / H, o = e % H;
-    store_bf16(smem + kW2T, core_offset(i, o, H), params[PW2 + o * H + i]);
+#pragma unroll
+  for (int e = tid; e < H * (H / 8); e += kThreads) {
+    const int i = e % H, o = e / H * 8;
+    float v[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = params[PW2 + (o + j) * H + i];
+    store8_bf16(smem + kW2T, core_offset(i, o, H), v);
   }
   for (int i = tid; i < H; i += kThreads) {
     b1[i] = params[PB1 + i];
@@ -400,11 +424,12 @@ __global__ void __launch_bounds__(kThreads, 1) k_mlp_train_tc(const __nv_bfloat1
   if (ok && lane == 0) atomicAdd(loss, upstream ? my_loss : my_loss / (6.0f * (float)n));
   if (ok) {
     // row tid of the accumulated gradients (columns per the buffers' features)
+    const bool wide = (reinterpret_cast<uintptr_t>(grad) & 15u) == 0;
     if (warp < 2) {  // rows 0..63: dW1 (columns 0..15), b1 (80), dW3^T (D2 columns 0..7)
       float v[16];
       tmem_ld16(tmem + lanes + kD1, v);
 #pragma unroll
-      for (int c = 0; c < IN; ++c) atomicAdd(&grad[PW1 + tid * IN + c], v[c]);
+      for (int c = 0; c < IN; c += 4) add4(&grad[PW1 + tid * IN + c], v + c, wide);
       tmem_ld16(tmem + lanes + kD1 + 80, v);
       atomicAdd(&grad[PB1 + tid], v[0]);
       tmem_ld16(tmem + lanes + kD2, v);
@@ -417,7 +442,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_mlp_train_tc(const __nv_bfloat1
         float v[16];
         tmem_ld16(tmem + lanes + kD1 + 16 + (uint32_t)c, v);
 #pragma unroll
-        for (int j = 0; j < 16; ++j) atomicAdd(&grad[PW2 + o * H + c + j], v[j]);
+        for (int j = 0; j < 16; j += 4) add4(&grad[PW2 + o * H + c + j], v + j, wide);
       }
       float v[16];
       tmem_ld16(tmem + lanes + kD1 + 80, v);

@@ -196,7 +196,7 @@ def _nvcc_shared(sources, out, extra=()):
 def build_core(force=False):
     out = os.path.join(LIB_DIR, CORE_NAME)
     srcs = [os.path.join(CSRC, "lbm_core.cu"), os.path.join(CSRC, "lbm_closure.cu"), os.path.join(CSRC, "lbm_domain.cu")]
-    deps = srcs + [os.path.join(CSRC, f) for f in ("lbm_common.cuh", "lbm_mlp.cuh")] + \
+    deps = srcs + [os.path.join(CSRC, f) for f in ("lbm_common.cuh", "lbm_mlp.cuh", "lbm_tc.cuh", "lbm_mlp_tc.cuh")] + \
         [os.path.join(INCLUDE, "lbm_gb300.h")]
     if not force and os.path.exists(out) and all(os.path.getmtime(out) >= os.path.getmtime(d) for d in deps):
         return out
