@@ -111,6 +111,7 @@ class Ensemble:
         self.total_nodes = int(sum(self.nodes))
         self.parity = 0
         self.nt = 0
+        self._stage_buf = None
         self._graphs = {}   # by (steps, parity of the first)
         self._tables = {}
         self.tile = tuple(tile) if tile is not None else autotune(self)
@@ -263,24 +264,41 @@ class Ensemble:
         runtime.check(self._core.lbm_stream_synchronize(self._stream))
 
     # ------------------------------------------------------------------ access
+    def _stage(self, nbytes):
+        """Device buffer of at least ``nbytes`` for moments on their way out (kept between calls)."""
+        if self._stage_buf is None or self._stage_buf.nbytes < nbytes:
+            if self._stage_buf is not None:
+                self.synchronize()
+                self._stage_buf.free()
+            self._stage_buf = runtime.DeviceBuffer(nbytes)
+        return self._stage_buf
+
     def moments(self, i, keys=None):
         """Interior moments (nv or len(keys), *shape) of instance ``i`` in float64."""
         lat, mlat, dom = self.lats[i], self.mlats[i], self.domains[i]
         es = runtime.DTYPE_SIZE[self.storage]
-        mbuf = runtime.DeviceBuffer(mlat.elements * 8)
-        f = ctypes.c_void_p(self.arena.ptr + self.offsets[i][self.parity] * es)
-        self.module.call(self.module.lib.lbm_f2m(f, ctypes.byref(lat), mbuf.handle, ctypes.byref(mlat), self._stream))
         keys = range(self.scheme.nv) if keys is None else keys
+        planes = [self.scheme.consm[k] if isinstance(k, (sp.Symbol, sp.IndexedBase)) else int(k) for k in keys]
+        f = ctypes.c_void_p(self.arena.ptr + self.offsets[i][self.parity] * es)
+        nc = self.scheme.nconsm
+        if planes and all(0 <= k < nc for k in planes):
+            # conserved moments only: one pass from the populations to a dense
+            # array of the interior, one copy to the host
+            out = np.empty([nc] + [int(n) for n in dom.shape_in])
+            stage = self._stage(out.nbytes)
+            self.module.call(self.module.lib.lbm_f2m_conserved_dense(f, ctypes.byref(lat), stage.handle, self._stream))
+            stage.download(out, stream=self._stream)
+            return out if planes == list(range(nc)) else out[planes]
+        mbuf = self._stage(mlat.elements * 8)
+        self.module.call(self.module.lib.lbm_f2m(f, ctypes.byref(lat), mbuf.handle, ctypes.byref(mlat), self._stream))
         out = []
         inner = tuple(slice(int(h), -int(h)) for h in dom.halo)
-        for k in keys:
-            k = self.scheme.consm[k] if isinstance(k, (sp.Symbol, sp.IndexedBase)) else int(k)
+        for k in planes:
             plane = np.empty(mlat.vstride)
             mbuf.download(plane, offset=k * mlat.vstride * 8, stream=self._stream)
             v = np.lib.stride_tricks.as_strided(plane[mlat.origin:], shape=dom.shape_halo,
                                                 strides=[mlat.stride[d] * 8 for d in range(dom.dim)])
             out.append(np.array(v[inner]))
-        mbuf.free()
         return np.array(out)
 
     def population_sums(self, i):
@@ -301,6 +319,9 @@ class Ensemble:
 
     def free(self):
         self._drop_graph()
+        if self._stage_buf is not None:
+            self._stage_buf.free()
+            self._stage_buf = None
         self.arena.free()
         for dinst, dtiles, _, _ in self._tables.values():
             dinst.free()

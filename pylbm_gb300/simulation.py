@@ -233,6 +233,8 @@ class Simulation:
         self.multi_step = True      # run() advances several steps per launch where the lattice allows it
         self._multi = {}            # (lbm_tile_plan, lbm_tile_boundary) by mode
         self._batch_entries = None  # links of the batched boundary launch, FP32 form, for the tiles
+        self._lat_ref = ctypes.byref(self._lat)
+        self._prm_array = None
         self._graphs = {}           # captured steps by what they launch
         self._graph_steps = 0       # steps run since the graphs were dropped
         self._need_init = True
@@ -264,6 +266,14 @@ class Simulation:
         if missing:
             raise ValueError(f"extra_parameters must give values for {missing}")
         return np.array([float(vals.get(n, 0.0)) for n in names] + [0.0], dtype=np.float64)
+
+    def _step_prm(self):
+        """Address of the run-time parameter vector of a step.  Without free
+        symbols it never changes; otherwise it follows ``extra_parameters``."""
+        if self._prm_array is None or self.scheme.free_symbols:
+            self._prm_array = self._prm()
+            self._prm_ptr = self._prm_array.ctypes.data
+        return self._prm_ptr
 
     def feq_host(self, cons):
         """Equilibrium populations of boundary values on the host.
@@ -385,6 +395,7 @@ class Simulation:
         self._upload_ghost()
         self._bc_batch = self._batch_table()
         self._walls = self._wall_table()
+        self._wall_ptrs = None if self._walls is None else tuple(a.ctypes.data for a in self._walls)
         self._multi = {}
         if self._multi_mode() == runtime.LBM_TILE_LINKS:
             self._multi_plan(runtime.LBM_TILE_LINKS)  # with the other lists, not in the first run
@@ -554,7 +565,7 @@ class Simulation:
 
     # ------------------------------------------------------------------ step
     def _enqueue_boundary(self, F):
-        lat = ctypes.byref(self._lat)
+        lat = self._lat_ref
         batch = self._bc_batch is not None and self.batch_boundary
         if self._full_halo:
             runtime.check(self._core.lbm_update_halo(F.handle, lat, self._stream))
@@ -563,7 +574,9 @@ class Simulation:
             runtime.check(self._core.lbm_boundary_batch(F.handle, lat, buf.handle, nmeth, total, self._stream))
         if batch:
             buf, nmeth, total = self._bc_batch
-            runtime.check(self._core.lbm_boundary_batch(F.handle, lat, buf.handle, nmeth, total, self._stream))
+            rc = self._core.lbm_boundary_batch(F.ptr, lat, buf.ptr, nmeth, total, self._stream)
+            if rc:
+                runtime.check(rc)
             return
         for meth, dev in self._bc_dev:
             il, st, rhs, ordered = dev["iload"], dev["istore"].handle, dev["rhs"].handle, dev["ordered"]
@@ -632,8 +645,11 @@ class Simulation:
                 model.norm_ptr(), model.guard_ptr(), model.rate_ptr(), self._fallbacks.handle, model.grid,
                 self._stream))
             return
-        fn = self.module.lib.lbm_one_time_step_periodic if self.periodic else self.module.lib.lbm_one_time_step
-        self.module.call(fn(F.handle, Fnew.handle, ctypes.byref(self._lat), pp, self._stream))
+        lib = self.module.lib
+        fn = lib.lbm_one_time_step_periodic if self.periodic else lib.lbm_one_time_step
+        rc = fn(F.ptr, Fnew.ptr, self._lat_ref, pp, self._stream)
+        if rc:
+            self.module.call(rc)
 
     def _closure_on_tensor_cores(self):
         kernel = getattr(self, "closure_kernel", "auto")
@@ -661,18 +677,18 @@ class Simulation:
         return self._walls is not None and self.fold_walls and getattr(self, "closure", None) is None
 
     def _launch_walls_step(self, F, Fnew, pp):
-        table, sym = self._walls
-        self.module.call(self.module.lib.lbm_one_time_step_walls(
-            F.handle, Fnew.handle, ctypes.byref(self._lat), pp, table.ctypes.data_as(ctypes.c_void_p),
-            sym.ctypes.data_as(ctypes.c_void_p), self._stream))
+        rc = self.module.lib.lbm_one_time_step_walls(F.ptr, Fnew.ptr, self._lat_ref, pp, *self._wall_ptrs, self._stream)
+        if rc:
+            self.module.call(rc)
 
     def _enqueue_step(self, F, Fnew, prm):
+        pp = prm.ctypes.data
         if self._folded():
-            self._launch_walls_step(F, Fnew, prm.ctypes.data_as(ctypes.c_void_p))
+            self._launch_walls_step(F, Fnew, pp)
             return
         if not self.periodic:
             self._enqueue_boundary(F)
-        self._launch_step(F, Fnew, prm.ctypes.data_as(ctypes.c_void_p))
+        self._launch_step(F, Fnew, pp)
 
     def boundary_condition(self):
         """Ghost refresh then every boundary method (pylbm/simulation.py:374-390)."""
@@ -699,15 +715,16 @@ class Simulation:
         self._update_m = True
         self._eq_pending = False
         self._m_cache = {}
-        prm = self._prm()
+        F, Fnew = self._F, self._Fnew
+        prm = self._step_prm()
         if self._folded():
-            self._launch_walls_step(self._F, self._Fnew, prm.ctypes.data_as(ctypes.c_void_p))
+            self._launch_walls_step(F, Fnew, prm)
         else:
             if not self.periodic:
                 self.boundary_condition()
-            self._launch_step(self._F, self._Fnew, prm.ctypes.data_as(ctypes.c_void_p))
-        self._F, self._Fnew = self._Fnew, self._F
-        self.t += self.dt
+            self._launch_step(F, Fnew, prm)
+        self._F, self._Fnew = Fnew, F
+        self.t += self._dt
         self.nt += 1
 
     # ---------------------------------------------------- phase by phase
