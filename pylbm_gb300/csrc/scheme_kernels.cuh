@@ -1904,9 +1904,12 @@ static int tile_grant(const char* who) {
 // lane-nodes a microsecond.  Where several blocks share an SM one's loads run
 // beside another's steps, and 0.6 (16 bits: 0.75) of the steps' time and 0.75 of the traffic's
 // at 5 TB/s remain.  Single steps stay (shape -1) where they are expected to be
-// no slower; for 16-bit storage, whose two-node step moves half the bytes,
-// from 1.5 10^6 nodes on (1536^2 FP16: 15.4 us a step against 15.6).
-inline void tile_rule(const lbm_lattice& lat, int& shape, int& margin) {
+// no slower: for 16-bit storage, whose two-node step moves half the bytes,
+// from 6 10^5 nodes on (FP16 periodic 700^2 5.5 us a step against 4.0 here,
+// 900^2 6.2 against 6.3), with box walls from 3 10^5 on (512^2 3.9 against
+// 3.7, 1024^2 8.0 against 9.4), and with boundary links, whose single step is
+// two launches, from 1.5 10^6 on.
+inline void tile_rule(const lbm_lattice& lat, int mode, int& shape, int& margin) {
   constexpr bool kHalf = sizeof(S) == 2;
   constexpr double kLaunchUs = 2.6, kRate = kHalf ? 1350.0 : 1600.0;
   int dev = 0, sms = 0;
@@ -1916,7 +1919,8 @@ inline void tile_rule(const lbm_lattice& lat, int& shape, int& margin) {
     sms = 152;
   }
   const double nodes = (double)lat.n[0] * lat.n[1];
-  double best = kHalf ? (nodes < 1.5e6 ? 1.9 + 6.0e-6 * nodes : 0.0) : kLaunchUs + 10e-6 * nodes;
+  const double most = mode == LBM_TILE_PERIODIC ? 6e5 : mode == LBM_TILE_WALLS ? 3e5 : 1.5e6;  // 16-bit storage
+  double best = kHalf ? (nodes < most ? 1.4 + 5.4e-6 * nodes : 0.0) : kLaunchUs + 10e-6 * nodes;
   shape = -1;
   for (int s = 0; s < kTileShapes; ++s)
     with_tile_shape(s, [&](auto tag) {
@@ -1971,13 +1975,15 @@ inline void plane_rule(const lbm_lattice& lat, bool walls, int shape, lbm_tile_p
     sms = 152;
   }
   const int n0 = lat.n[0], n1 = lat.n[1], n2 = lat.n[2];
-  // Expected microseconds: two single steps, 2.8 and the traffic at 6.5 TB/s
-  // each; a two-step launch, 2.5 and 2 more a wave, for every plane of a block
+  // Expected microseconds: two single steps, 2 and the traffic at 6.5 TB/s
+  // (7.2 from L2) each, less what the walk has to be better by; a two-step launch, 2.5 and 2 more a wave, for every plane of a block
   // 0.35 and 0.045 a warp and step (19 populations; short rows, read in part
   // sectors, cost more, and so do rows that end at walls: with one wave the
   // blocks at the walls set the time, with several they are shared out).  D3Q19 FP32 at 24^3 to 256^3 keeps to
   // it within 12 %.
-  double best = shape >= 0 ? 1e30 : (walls ? 0.90 : 0.97) * 2.0 * (2.8 + (double)n0 * n1 * n2 * 2 * LBM_Q * sizeof(S) / 6.5e6);
+  const double bytes = (double)n0 * n1 * n2 * 2 * LBM_Q * sizeof(S);
+  const bool cached = bytes < 100e6;  // both buffers stay in L2
+  double best = shape >= 0 ? 1e30 : (cached ? 0.86 : walls ? 0.90 : 0.95) * 2.0 * (2.0 + bytes / (cached ? 7.2e6 : 6.5e6));
   const double warp_us = 0.045 * LBM_Q / 19;
   for (int t2 = (n2 + kPlaneSlack - 4) / (kPlaneSlack - 3); t2 <= n2; ++t2) {
     const int o2 = (n2 + t2 - 1) / t2, most = kPlaneThreads / (o2 + 2) - 2;
@@ -2027,7 +2033,7 @@ extern "C" int lbm_scheme_multi_step_plan(const lbm_lattice* lat, int32_t mode, 
   if (lat->elements >= (1LL << 31)) return LBM_OK;  // the kernel indexes with 32 bits
   if (shape >= kTileShapes) return lbm::fail(LBM_ERR_ARG, "%s: shape %d", who, shape);
   if (shape < 0) {
-    tile_rule(*lat, shape, margin);
+    tile_rule(*lat, mode, shape, margin);
     if (shape < 0) return LBM_OK;
   }
   return with_tile_shape(shape, [&](auto tag) {
