@@ -1995,9 +1995,11 @@ inline void plane_rule(const lbm_lattice& lat, bool walls, int shape, lbm_tile_p
       for (int t0 = 1; t0 <= (n0 + 3) / 4; ++t0) {
         const int planes = (n0 + t0 - 1) / t0;
         if (shape >= 0 && planes != shape) continue;
-        const double waves = (double)(((long long)t0 * t1 * t2 + sms - 1) / sms);
+        const double blocks = (double)t0 * t1 * t2;
+        double waves = (double)(((long long)blocks + sms - 1) / sms);
+        if (walls && waves > 1.0) waves = blocks / sms + 0.6;  // blocks of unequal cost
         const double warps = (planes + 2) * first + planes * second;
-        const double row = !walls ? 1.0 + 3.0 / o2 : waves > 1.0 ? 1.18 * (1.0 + 5.0 / o2) : 1.2 * (1.0 + 6.0 / o2);
+        const double row = !walls ? 1.0 + 3.0 / o2 : (waves > 1.0 ? 1.05 : 1.22) * (1.0 + 4.0 / o2) * (o2 % 32 ? 1.08 : 1.0);
         const double us = 0.5 + waves * (2.0 + (planes + 2) * 0.35 + row * warp_us * warps);
         if (us >= best) continue;
         best = us;

@@ -104,6 +104,31 @@ def test_two_steps_3d_equal_single_steps(box):
         sim.free()
 
 
+@pytest.mark.parametrize("walls", [False, True])
+def test_two_steps_3d_columns(walls):
+    """Columns of the narrowest and widest cross-sections a block can hold."""
+    from pylbm_gb300 import runtime
+
+    n = (9, 64, 75)
+    c0 = [1.0, 0.0, 0.0, 0.0]
+    single = Simulation(_box3d(n, walls), dtype="float32", c0=c0)
+    single.multi_step = False
+    single.run(8)
+    ref = _populations(single)
+    single.free()
+    for out in ((7, 69), (62, 8), (8, 57), (18, 30), (9, 55), (1, 1)):
+        sim = Simulation(_box3d(n, walls), dtype="float32", c0=c0)
+        mode = sim._multi_mode()
+        plan, bnd = sim._multi_plan(mode, 5, 0)
+        plan = runtime.TilePlan.from_buffer_copy(plan)
+        for d in range(2):
+            plan.out[d], plan.tiles[d] = out[d], -(-n[1 + d] // out[d])
+        sim._multi[mode] = (plan, bnd)
+        sim.run(8)
+        assert np.array_equal(_populations(sim), ref), out
+        sim.free()
+
+
 def test_captured_launches_continue_the_run():
     runs = []
     for multi in (True, False):
