@@ -251,6 +251,7 @@ __global__ void __launch_bounds__(kPlaneThreads, 1) k_two_steps(const S* __restr
   }
   const int i1 = o1 + r, i2 = o2 + c;
   t.active = used && r < a.out1 + 2 && i1 <= a.n[1] && i2 <= a.n[2];
+  if (kWalls) t.active = t.active && i1 >= 0 && i1 < a.n[1] && i2 >= 0 && i2 < a.n[2];
   t.inside = t.active && r >= 1 && r <= a.out1 && c >= 1 && c <= a.out2 && i1 < a.n[1] && i2 < a.n[2];
   t.below1 = i1 == 0 ? -3 : 0;
   t.above1 = i1 == a.n[1] - 1 ? 3 : 0;
