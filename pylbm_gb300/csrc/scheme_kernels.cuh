@@ -1346,23 +1346,27 @@ inline dim3 node_grid(const lbm_lattice& l, bool with_halo) {
   return dim3(gx, gy, gz);
 }
 
-// Threads of a step block along a row of `work` nodes (or node pairs): as few
-// idle lanes as 32, 64, 96 or 128 threads allow, then the largest block.  A
-// row of 96 pairs in blocks of 128 left a quarter of the registers to warps
-// without work (D3Q19 FP16 192^3: 102 us a step).  FP64 takes 64 threads where
-// it can: its steps are bound by the FP64 pipe of the busiest SM, and
-// 256^2 nodes are 13.5 warps an SM, 14 at most in blocks of two warps against
-// 16 in blocks of four (25.8 us a step).
+// Threads of a step block along a row of `work` nodes (or node pairs).  A row
+// that one or two warps cover takes them alone; longer ones 128 threads, or 96
+// where that leaves an eighth fewer idle lanes: rows of 96 pairs in blocks of
+// 128 left a quarter of the registers to warps without work (D3Q19 FP16 192^3:
+// 102 us a step against 96), while blocks of one or two warps cost more than
+// they save on long rows (D2Q9 BF16 778^2: 6.6 us a step in blocks of 32
+// threads, 5.3 in 128).  FP64 takes what idles least, and 64 threads before
+// 128: its steps are bound by the FP64 pipe of the busiest SM, and 256^2 nodes
+// are 13.5 warps an SM, 14 at most in blocks of two warps against 16 in blocks
+// of four (20.5 against 25.8 us a step; 160^2 9.7 in blocks of 32 threads,
+// 16.3 in 128).
 inline unsigned step_block(int work) {
-  unsigned best = 0, waste = 0;
-  for (unsigned b = LBM_BLOCK; b >= 32; b -= 32) {
-    const unsigned w = ((unsigned)work + b - 1) / b * b - (unsigned)work;
-    if (best == 0 || w < waste || (w == waste && sizeof(S) == 8 && b == 64)) {
-      best = b;
-      waste = w;
-    }
+  const auto lanes = [&](unsigned b) { return ((unsigned)work + b - 1) / b * b; };
+  if (sizeof(S) == 8) {
+    unsigned best = 64;
+    for (unsigned b = 128; b >= 32; b -= 32)
+      if (lanes(b) < lanes(best)) best = b;
+    return best;
   }
-  return best;
+  if (work <= 64) return work <= 32 ? 32 : 64;
+  return 8 * lanes(96) <= 7 * lanes(128) ? 96 : 128;
 }
 
 // Two-node words need every pair (z, z+1), z even, on a 4-byte boundary: even
