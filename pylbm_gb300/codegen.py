@@ -731,7 +731,7 @@ class SchemeSource:
                 + ("#define LBM_FLOAT_COMPUTE 1\n" if compute == "float32" else "")
                 + ("#define LBM_PLANE_STEPS 1\n" if storage == "float32" and not self.absolute_collide else "") +
                 "#include \"lbm_common.cuh\"\n"
-                "using lbm::lbm_fma;\nusing lbm::lbm_neg;\n"
+                "using lbm::lbm_fma;\nusing lbm::lbm_scaled_add;\nusing lbm::lbm_neg;\n"
                 "template <typename R> __device__ __forceinline__ R lbm_sqrt(R x) { return sqrt(x); }\n"
                 "template <typename R> __device__ __forceinline__ R lbm_pow(R x, R e) { return pow(x, e); }\n"
                 + self.header() +

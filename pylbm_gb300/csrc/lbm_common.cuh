@@ -145,6 +145,13 @@ __device__ __forceinline__ F2 lbm_fma<F2>(F2 a, F2 b, F2 c) {
   return r;
 }
 
+// p*a + b for a power of two p: the product is exact, so one multiply-add
+// rounds once, exactly as the printed multiply and add do.
+template <typename R>
+__device__ __forceinline__ R lbm_scaled_add(R p, R a, R b) {
+  return lbm_fma<R>(p, a, b);
+}
+
 // -a; in FP64 as a flip of the sign bit, which the FP64 pipe has no part in (a
 // negation on its own is an addition there)
 template <typename R>

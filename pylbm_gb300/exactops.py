@@ -77,7 +77,7 @@ class _Program:
         if abs(s) != 1.0 and (abs(t) == 1.0 or abs(t) > abs(s)):  # the sum keeps a scale of one where it can
             (s, a), (t, b) = (t, b), (s, a)
         r = t / s
-        return (s, self._base(("add", a, r, b), f"lbm_fma<R>(LBM_R({r!r}), {self.names[b]}, {self.names[a]})", "fma"))
+        return (s, self._base(("add", a, r, b), f"lbm_scaled_add<R>(LBM_R({r!r}), {self.names[b]}, {self.names[a]})", "fma"))
 
     def value(self, v):
         """C expression of a scaled value."""

@@ -18,7 +18,7 @@ def _fma(a, b, c):
 
 def _run(lines, env):
     for line in lines:
-        text = line.strip().rstrip(";").replace("const R ", "").replace("lbm_fma<R>", "_fma").replace("lbm_neg<R>", "-")
+        text = line.strip().rstrip(";").replace("const R ", "").replace("lbm_scaled_add<R>", "_fma").replace("lbm_neg<R>", "-")
         exec(re.sub(r"LBM_R\(([^()]*)\)", r"(\1)", text), {"_fma": _fma, "pow": math.pow}, env)
 
 
