@@ -235,7 +235,8 @@ class Simulation:
         self._batch_entries = None  # links of the batched boundary launch, FP32 form, for the tiles
         self._lat_ref = ctypes.byref(self._lat)
         self._prm_array = None
-        self._graphs = {}           # captured steps by what they launch
+        self.launches = 0           # step and boundary kernels put on the stream so far
+        self._graphs = {}           # captured steps by what they launch: (graph, its kernels)
         self._graph_steps = 0       # steps run since the graphs were dropped
         self._need_init = True
         if initialize:
@@ -660,7 +661,8 @@ class Simulation:
         return kernel == "tc"
 
     def launches_per_step(self):
-        """Kernel launches of one step: ghost refresh, boundary methods, step."""
+        """Kernel launches of one step taken singly: ghost refresh, boundary methods,
+        step (``launches`` counts what was put on the stream)."""
         if self.periodic or self._folded():
             return 1
         batch = self._bc_batch is not None and self.batch_boundary
@@ -683,6 +685,7 @@ class Simulation:
 
     def _enqueue_step(self, F, Fnew, prm):
         pp = prm.ctypes.data
+        self.launches += self.launches_per_step()
         if self._folded():
             self._launch_walls_step(F, Fnew, pp)
             return
@@ -726,6 +729,7 @@ class Simulation:
         self._F, self._Fnew = Fnew, F
         self.t += self._dt
         self.nt += 1
+        self.launches += 1 if self.periodic else self.launches_per_step()
 
     # ---------------------------------------------------- phase by phase
     # pylbm's routines for users who split the step themselves
@@ -863,7 +867,7 @@ class Simulation:
         self._m_partial = False
 
     def _drop_graph(self):
-        for graph in self._graphs.values():
+        for graph, _ in self._graphs.values():
             self._core.lbm_graph_destroy(graph)
         self._graphs = {}
         self._graph_steps = 0
@@ -936,6 +940,8 @@ class Simulation:
         self.module.call(self.module.lib.lbm_scheme_multi_step(
             self._F.handle, self._Fnew.handle, ctypes.byref(self._lat), prm.ctypes.data_as(ctypes.c_void_p),
             ctypes.byref(plan), steps, mode, ctypes.byref(bnd), self._stream))
+        # an even number of launches in 2D, of two steps each in 3D
+        self.launches += steps // 2 if self.dim == 3 else 2 * -(-steps // (2 * plan.margin))
 
     def _enqueue_steps(self, prm, steps):
         """An even number of steps, one launch sequence each, from F back to F."""
@@ -953,16 +959,20 @@ class Simulation:
         key = (kind, unit, self._F.ptr, self._Fnew.ptr, tuple(prm))
         if steps < unit:
             return 0
-        graph = self._graphs.get(key)
-        if graph is None:
+        if key not in self._graphs:
             self._graph_steps += steps
             if not always and self._graph_steps < 2 * unit:
                 return 0
             if len(self._graphs) >= 4:
                 self._drop_graph()
-            graph = self._graphs[key] = self._capture(lambda: enqueue(unit))
+            before = self.launches
+            graph = self._capture(lambda: enqueue(unit))
+            self._graphs[key] = (graph, self.launches - before)
+            self.launches = before
+        graph, kernels = self._graphs[key]
         for _ in range(steps // unit):
             runtime.check(self._core.lbm_graph_launch(graph, self._stream))
+        self.launches += steps // unit * kernels
         return steps // unit * unit
 
     def _capture(self, enqueue):
