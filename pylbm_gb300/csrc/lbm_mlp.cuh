@@ -189,4 +189,79 @@ __device__ __forceinline__ void forward_tile(const uint32_t (&xa)[4], const __nv
   }
 }
 
+// Forward pass of kTiles 16-row tiles side by side, the values of
+// forward_tile for each: every weight fragment and bias is loaded once for all
+// tiles, and their MMA and tanh chains fill one another's latency.  A hidden
+// layer is made in pairs of output tiles, each packed at once into an A
+// fragment; the second layer's goes straight into the output, so that the
+// first layer's activations are all that is kept.
+template <int kTiles>
+__device__ __forceinline__ void forward_tiles(const uint32_t (&xa)[kTiles][4], const __nv_bfloat16* __restrict__ wb,
+                                              const float* __restrict__ b1, const float* __restrict__ b2,
+                                              const float* __restrict__ b3, int lane, float (&y)[kTiles][4]) {
+  const int t = lane & 3;
+  uint32_t h1a[kTiles][4][4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    float acc[kTiles][2][4];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int nt = 2 * j + i;
+      const float2 c = *reinterpret_cast<const float2*>(b1 + nt * 8 + 2 * t);
+      uint32_t bb0, bb1;
+      load_b(wb + BW1T, IN, nt, 0, lane, bb0, bb1);
+#pragma unroll
+      for (int u = 0; u < kTiles; ++u) {
+        acc[u][i][0] = acc[u][i][2] = c.x;
+        acc[u][i][1] = acc[u][i][3] = c.y;
+        mma16816(acc[u][i], xa[u], bb0, bb1);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kTiles; ++u) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) acc[u][i >> 2][i & 3] = silu(acc[u][i >> 2][i & 3]);
+      d_to_a(acc[u][0], acc[u][1], h1a[u][j]);
+    }
+  }
+  const float2 c3 = *reinterpret_cast<const float2*>(b3 + 2 * t);
+#pragma unroll
+  for (int u = 0; u < kTiles; ++u) {
+    y[u][0] = y[u][2] = c3.x;
+    y[u][1] = y[u][3] = c3.y;
+  }
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    float acc[kTiles][2][4];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const float2 c = *reinterpret_cast<const float2*>(b2 + (2 * j + i) * 8 + 2 * t);
+#pragma unroll
+      for (int u = 0; u < kTiles; ++u) {
+        acc[u][i][0] = acc[u][i][2] = c.x;
+        acc[u][i][1] = acc[u][i][3] = c.y;
+      }
+    }
+#pragma unroll
+    for (int kt = 0; kt < 4; ++kt)
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        uint32_t bb0, bb1;
+        load_b(wb + BW2T, H, 2 * j + i, kt, lane, bb0, bb1);
+#pragma unroll
+        for (int u = 0; u < kTiles; ++u) mma16816(acc[u][i], h1a[u][kt], bb0, bb1);
+      }
+    uint32_t b30, b31;
+    load_b(wb + BW3T, H, 0, j, lane, b30, b31);
+#pragma unroll
+    for (int u = 0; u < kTiles; ++u) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) acc[u][i >> 2][i & 3] = silu(acc[u][i >> 2][i & 3]);
+      uint32_t h2a[4];
+      d_to_a(acc[u][0], acc[u][1], h2a);
+      mma16816(y[u], h2a, b30, b31);
+    }
+  }
+}
+
 }  // namespace lbm_mlp

@@ -107,6 +107,11 @@ __global__ void __launch_bounds__(LBM_BLOCK) k_step_ghost(const S* __restrict__ 
   for (int k = 0; k < LBM_Q; ++k) Store<S>::store(fnew + o + (long long)k * a.g.vstride, g[k]);
 }
 
+template <typename T>
+__device__ __forceinline__ T* byte_at(T* base, unsigned offset) {
+  return reinterpret_cast<T*>(reinterpret_cast<uintptr_t>(base) + offset);
+}
+
 // offset of the pulled neighbour along one axis, wrapped into the interior
 __device__ __forceinline__ long long wrap_off(int i, int s, int n, int h, long long stride) {
   int j = i - s;
@@ -309,11 +314,6 @@ __device__ __forceinline__ long long pair_row(const Geo& g, int i0, int i1) {
 #else
   return g.origin + (long long)i0 * g.stride[0] + (long long)i1 * g.stride[1] + g.h[2] - 2;
 #endif
-}
-
-template <typename T>
-__device__ __forceinline__ T* byte_at(T* base, unsigned offset) {
-  return reinterpret_cast<T*>(reinterpret_cast<uintptr_t>(base) + offset);
 }
 
 // pulled pair of a population row, velocity component vl along the contiguous axis
@@ -780,7 +780,9 @@ __global__ void __launch_bounds__(LBM_ENSEMBLE_MAX_BLOCK, !LBM_HAS_PAIRS ? 0 : L
 // non-conserved moments receive the MLP's correction, computed from the
 // node's pre-collision moments.  Each warp stages the normalised moments of
 // its 32 nodes in shared memory and evaluates the MLP on the tensor cores as
-// two 16-row tiles (lbm_mlp.cuh); conserved moments are never changed.
+// two 16-row tiles side by side (lbm_mlp.cuh); conserved moments are never
+// changed.  One tile after the other, and 64-bit places: 8.27 us a step at
+// 256^2, 20.9 at 512^2, 43.8 at 768^2; now 8.02, 19.4, 40.0.
 struct ClosureArgs {
   const __nv_bfloat16* w;  // BF16 weight block (forward part read)
   const float* params;     // FP32 parameter block (biases read)
@@ -809,6 +811,54 @@ __device__ __forceinline__ float closure_correction(const ClosureArgs& c, int j,
   return lam * d;
 }
 
+// What the closure steps (one thread per node of the interior, numbered along
+// its rows) do with the node's number and place.  kNarrow: a population spans
+// less than 2^32 bytes, so that its number divides and its offsets add in 32
+// bits, to a base per population that all lanes share: the steps are bound by
+// instructions from 384^2 on (768^2: 41.5 us with 64 bits, 40.0 with 32; the
+// tensor-memory step at 1024^2: 70.8 and 68.6).
+template <bool kNarrow>
+struct ClosurePlace {
+  using Count = std::conditional_t<kNarrow, unsigned, unsigned long long>;
+  using Offset = std::conditional_t<kNarrow, int, long long>;
+  int idx[3];
+  Offset own;  // elements from population 0
+  __device__ __forceinline__ ClosurePlace(const Geo& g, long long node) : idx{0, 0, 0} {
+    Count q = (Count)node;
+#pragma unroll
+    for (int d = LBM_DIM - 1; d > 0; --d) {
+      const Count r = q / (Count)g.n[d];
+      idx[d] = (int)(q - r * (Count)g.n[d]) + g.h[d];
+      q = r;
+    }
+    idx[0] = (int)q + g.h[0];
+    own = (Offset)lbm::node_offset(g, idx[0], idx[1], idx[2]);
+  }
+  template <typename T>
+  __device__ __forceinline__ static T* at(T* f, const Geo& g, int k, Offset e) {
+    if constexpr (kNarrow) return byte_at(f + (long long)k * g.vstride, (unsigned)e * (unsigned)sizeof(T));
+    return f + e + (long long)k * g.vstride;
+  }
+  __device__ __forceinline__ void pull(const S* __restrict__ f, const Geo& g, R* gv) const {
+    Offset off0[2 * LBM_VMAX + 1], off1[2 * LBM_VMAX + 1], off2[2 * LBM_VMAX + 1];
+#pragma unroll
+    for (int s = -LBM_VMAX; s <= LBM_VMAX; ++s) {
+      off0[s + LBM_VMAX] = LBM_DIM > 0 ? (Offset)wrap_off(idx[0], s, g.n[0], g.h[0], g.stride[0]) : 0;
+      off1[s + LBM_VMAX] = LBM_DIM > 1 ? (Offset)wrap_off(idx[1], s, g.n[1], g.h[1], g.stride[1]) : 0;
+      off2[s + LBM_VMAX] = LBM_DIM > 2 ? (Offset)wrap_off(idx[2], s, g.n[2], g.h[2], g.stride[2]) : 0;
+    }
+#define LBM_PULL_CL(k, vx, vy, vz)                                                                     \
+  gv[k] = (R)Store<S>::load(at(f, g, k, own + off0[(vx) + LBM_VMAX] + off1[(vy) + LBM_VMAX] +          \
+                                            off2[(vz) + LBM_VMAX]));
+    LBM_FOR_EACH_V(LBM_PULL_CL)
+#undef LBM_PULL_CL
+  }
+  __device__ __forceinline__ void store(S* __restrict__ fnew, const Geo& g, const R* gv) const {
+#pragma unroll
+    for (int k = 0; k < LBM_Q; ++k) Store<S>::store(at(fnew, g, k, own), gv[k]);
+  }
+};
+
 constexpr int kClosureWarps = 8;
 // nodes per warp and pass: 32 (every lane pulls, relaxes and stores a node;
 // the MLP runs as two 16-row tiles) or 16 (lanes 16..31 only join the MLP)
@@ -818,10 +868,12 @@ constexpr int kClosureWarps = 8;
 constexpr int kClosureWarpNodes = LBM_CLOSURE_WARP_NODES;
 static_assert(kClosureWarpNodes == 16 || kClosureWarpNodes == 32, "16 or 32 nodes per warp");
 #ifndef LBM_CLOSURE_MIN_BLOCKS
-// no register cap: capping at 64 or 80 registers spills and was slower
-#define LBM_CLOSURE_MIN_BLOCKS 1
+// 128 registers: without a cap both tiles' activations take 168, and the second
+// block of an SM waits (256^2: 10.3 us a step); 80 spill (8.9)
+#define LBM_CLOSURE_MIN_BLOCKS 2
 #endif
 
+template <bool kNarrow>
 __global__ void __launch_bounds__(32 * kClosureWarps, LBM_CLOSURE_MIN_BLOCKS) k_step_periodic_closure(const S* __restrict__ f,
                                                                                S* __restrict__ fnew, StepArgs a,
                                                                                ClosureArgs c) {
@@ -855,33 +907,16 @@ __global__ void __launch_bounds__(32 * kClosureWarps, LBM_CLOSURE_MIN_BLOCKS) k_
   const int gq = lane >> 2, tq = lane & 3;
   const Geo& g = a.g;
   // kClosureWarpNodes nodes per warp: lane l owns node l of the warp's run
-  // (l < kClosureWarpNodes); all 32 lanes evaluate the MLP, one 16-row MMA
-  // tile after the other
+  // (l < kClosureWarpNodes); all 32 lanes evaluate the MLP of its 16-row MMA
+  // tiles
   const long long per_block = kClosureWarpNodes * (blockDim.x >> 5);
   for (long long base = (long long)blockIdx.x * per_block; base < c.nodes; base += (long long)gridDim.x * per_block) {
     const long long node = base + warp * kClosureWarpNodes + lane;
     const bool active = lane < kClosureWarpNodes && node < c.nodes;
-    int idx[3] = {0, 0, 0};
-    long long q = active ? node : 0;
-    for (int d = LBM_DIM - 1; d >= 0; --d) {
-      idx[d] = (int)(q % g.n[d]) + g.h[d];
-      q /= g.n[d];
-    }
-    const long long o = lbm::node_offset(g, idx[0], idx[1], idx[2]);
+    const ClosurePlace<kNarrow> place(g, active ? node : 0);
     R gv[LBM_Q], m[LBM_Q];
     if (active) {
-      long long off0[2 * LBM_VMAX + 1], off1[2 * LBM_VMAX + 1], off2[2 * LBM_VMAX + 1];
-#pragma unroll
-      for (int s = -LBM_VMAX; s <= LBM_VMAX; ++s) {
-        off0[s + LBM_VMAX] = LBM_DIM > 0 ? wrap_off(idx[0], s, g.n[0], g.h[0], g.stride[0]) : 0;
-        off1[s + LBM_VMAX] = LBM_DIM > 1 ? wrap_off(idx[1], s, g.n[1], g.h[1], g.stride[1]) : 0;
-        off2[s + LBM_VMAX] = LBM_DIM > 2 ? wrap_off(idx[2], s, g.n[2], g.h[2], g.stride[2]) : 0;
-      }
-#define LBM_PULL_CL(k, vx, vy, vz)                                                              \
-  gv[k] = (R)Store<S>::load(f + o + (long long)(k) * g.vstride + off0[(vx) + LBM_VMAX] +        \
-                            off1[(vy) + LBM_VMAX] + off2[(vz) + LBM_VMAX]);
-      LBM_FOR_EACH_V(LBM_PULL_CL)
-#undef LBM_PULL_CL
+      place.pull(f, g, gv);
       lbm_moments<R>(gv, m);
     } else {
 #pragma unroll
@@ -905,22 +940,25 @@ __global__ void __launch_bounds__(32 * kClosureWarps, LBM_CLOSURE_MIN_BLOCKS) k_
     } else {
       __syncwarp();
     }
-#pragma unroll 1
-    for (int t = 0; t < kClosureWarpNodes / 16; ++t) {
+    constexpr int kTiles = kClosureWarpNodes / 16;
+    uint32_t xa[kTiles][4];
+    float y[kTiles][4];
+#pragma unroll
+    for (int t = 0; t < kTiles; ++t) {
       const __nv_bfloat16* xt = &x_s[warp][t * 16 * IN];
-      uint32_t xa[4];
-      xa[0] = *reinterpret_cast<const uint32_t*>(xt + gq * IN + 2 * tq);
-      xa[1] = *reinterpret_cast<const uint32_t*>(xt + (gq + 8) * IN + 2 * tq);
-      xa[2] = *reinterpret_cast<const uint32_t*>(xt + gq * IN + 8 + 2 * tq);
-      xa[3] = *reinterpret_cast<const uint32_t*>(xt + (gq + 8) * IN + 8 + 2 * tq);
-      float y[4], z1[8][4], z2[8][4];
-      uint32_t h1a[4][4], h2a[4][4];
-      forward_tile<false>(xa, w_s, b_s, b_s + H, b_s + 2 * H, lane, y, z1, z2, h1a, h2a);
+      xa[t][0] = *reinterpret_cast<const uint32_t*>(xt + gq * IN + 2 * tq);
+      xa[t][1] = *reinterpret_cast<const uint32_t*>(xt + (gq + 8) * IN + 2 * tq);
+      xa[t][2] = *reinterpret_cast<const uint32_t*>(xt + gq * IN + 8 + 2 * tq);
+      xa[t][3] = *reinterpret_cast<const uint32_t*>(xt + (gq + 8) * IN + 8 + 2 * tq);
+    }
+    forward_tiles<kTiles>(xa, w_s, b_s, b_s + H, b_s + 2 * H, lane, y);
+#pragma unroll
+    for (int t = 0; t < kTiles; ++t) {
       float* yt = &y_s[warp][t * 16 * OUT];
-      yt[gq * OUT + 2 * tq] = y[0];
-      yt[gq * OUT + 2 * tq + 1] = y[1];
-      yt[(gq + 8) * OUT + 2 * tq] = y[2];
-      yt[(gq + 8) * OUT + 2 * tq + 1] = y[3];
+      yt[gq * OUT + 2 * tq] = y[t][0];
+      yt[gq * OUT + 2 * tq + 1] = y[t][1];
+      yt[(gq + 8) * OUT + 2 * tq] = y[t][2];
+      yt[(gq + 8) * OUT + 2 * tq + 1] = y[t][3];
     }
     __syncwarp();
     if (active) {
@@ -949,8 +987,7 @@ __global__ void __launch_bounds__(32 * kClosureWarps, LBM_CLOSURE_MIN_BLOCKS) k_
         atomicAdd(c.fallbacks, 1);
       }
       lbm_populations<R>(m, gv);
-#pragma unroll
-      for (int k = 0; k < LBM_Q; ++k) Store<S>::store(fnew + o + (long long)k * g.vstride, gv[k]);
+      place.store(fnew, g, gv);
     }
     __syncwarp();
   }
@@ -983,6 +1020,7 @@ struct ClosureTcSmem {
   uint32_t tmem_base;
 };
 
+template <bool kNarrow>
 __global__ void __launch_bounds__(kTcRows) k_step_periodic_closure_tc(const S* __restrict__ f, S* __restrict__ fnew,
                                                                      StepArgs a, ClosureArgs c) {
   using namespace lbm_mlp;
@@ -1021,27 +1059,10 @@ __global__ void __launch_bounds__(kTcRows) k_step_periodic_closure_tc(const S* _
   for (long long tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
     const long long node = tile * kTcRows + tid;
     const bool active = node < c.nodes;
-    int idx[3] = {0, 0, 0};
-    long long q = active ? node : 0;
-    for (int d = LBM_DIM - 1; d >= 0; --d) {
-      idx[d] = (int)(q % g.n[d]) + g.h[d];
-      q /= g.n[d];
-    }
-    const long long o = lbm::node_offset(g, idx[0], idx[1], idx[2]);
+    const ClosurePlace<kNarrow> place(g, active ? node : 0);
     R gv[LBM_Q], m[LBM_Q];
     if (active) {
-      long long off0[2 * LBM_VMAX + 1], off1[2 * LBM_VMAX + 1], off2[2 * LBM_VMAX + 1];
-#pragma unroll
-      for (int s = -LBM_VMAX; s <= LBM_VMAX; ++s) {
-        off0[s + LBM_VMAX] = LBM_DIM > 0 ? wrap_off(idx[0], s, g.n[0], g.h[0], g.stride[0]) : 0;
-        off1[s + LBM_VMAX] = LBM_DIM > 1 ? wrap_off(idx[1], s, g.n[1], g.h[1], g.stride[1]) : 0;
-        off2[s + LBM_VMAX] = LBM_DIM > 2 ? wrap_off(idx[2], s, g.n[2], g.h[2], g.stride[2]) : 0;
-      }
-#define LBM_PULL_TC(k, vx, vy, vz)                                                              \
-  gv[k] = (R)Store<S>::load(f + o + (long long)(k) * g.vstride + off0[(vx) + LBM_VMAX] +        \
-                            off1[(vy) + LBM_VMAX] + off2[(vz) + LBM_VMAX]);
-      LBM_FOR_EACH_V(LBM_PULL_TC)
-#undef LBM_PULL_TC
+      place.pull(f, g, gv);
       lbm_moments<R>(gv, m);
     } else {
 #pragma unroll
@@ -1126,8 +1147,7 @@ __global__ void __launch_bounds__(kTcRows) k_step_periodic_closure_tc(const S* _
         atomicAdd(c.fallbacks, 1);
       }
       lbm_populations<R>(m, gv);
-#pragma unroll
-      for (int k = 0; k < LBM_Q; ++k) Store<S>::store(fnew + o + (long long)k * g.vstride, gv[k]);
+      place.store(fnew, g, gv);
     }
     fence_before_sync();
     __syncthreads();
@@ -1450,7 +1470,7 @@ static int closure_tc_blocks_per_sm(int dev, int* used, int* bound_out) {
     const char* who = "closure_tc_blocks_per_sm";
     cudaFuncAttributes fa;
     int regs = 0, smem = 0, reserved = 0, threads = 0;
-    int rc = lbm::cuda_check(cudaFuncGetAttributes(&fa, lbm_scheme::k_step_periodic_closure_tc), who);
+    int rc = lbm::cuda_check(cudaFuncGetAttributes(&fa, lbm_scheme::k_step_periodic_closure_tc<true>), who);
     if (!rc) rc = lbm::cuda_check(cudaDeviceGetAttribute(&regs, cudaDevAttrMaxRegistersPerMultiprocessor, dev), who);
     if (!rc)
       rc = lbm::cuda_check(cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev), who);
@@ -1777,6 +1797,7 @@ static int closure_common(const void* f, void* fnew, const lbm_lattice* lat, con
       return lbm::fail(LBM_ERR_ARG, "%s: rate bounds of output %d: [%g, %g] (need -1 <= lo <= hi)", who, i,
                        (double)c.lam_lo[i], (double)c.lam_hi[i]);
   }
+  const bool narrow = (unsigned long long)lat->vstride * sizeof(S) < (1ULL << 32);
 #if LBM_Q <= 16 && (LBM_Q - LBM_NCONS) <= 8
   if (tc) {
     int dev = 0, sms = 0;
@@ -1789,13 +1810,14 @@ static int closure_common(const void* f, void* fnew, const lbm_lattice* lat, con
     const long long tiles = (c.nodes + kTcRows - 1) / kTcRows;
     const long long cap = (long long)per_sm * sms;
     const long long blocks = tiles < cap ? tiles : cap;
-    k_step_periodic_closure_tc<<<(unsigned)blocks, kTcRows, 0, (cudaStream_t)stream>>>((const S*)f, (S*)fnew, a, c);
+    auto* kernel = narrow ? k_step_periodic_closure_tc<true> : k_step_periodic_closure_tc<false>;
+    kernel<<<(unsigned)blocks, kTcRows, 0, (cudaStream_t)stream>>>((const S*)f, (S*)fnew, a, c);
     return lbm::launch_check(who);
   }
 #endif
   // Eight warps a block, which share the staged weights; fewer where that
-  // would leave SMs without a block (128^2 nodes: 6.2 us a step in blocks of
-  // four warps, 7.2 in blocks of eight)
+  // would leave SMs without a block (128^2 nodes, in graphs of two steps: 6.2
+  // us a step in blocks of four warps, 7.2 in blocks of eight; 4.4 now)
   int dev = 0, sms = 0;
   rc = lbm::cuda_check(cudaGetDevice(&dev), who);
   if (!rc) rc = lbm::cuda_check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), who);
@@ -1805,8 +1827,8 @@ static int closure_common(const void* f, void* fnew, const lbm_lattice* lat, con
   const int width = spread >= kClosureWarps ? kClosureWarps : spread < 4 ? 4 : (int)spread;
   long long blocks = (warps + width - 1) / width;
   if (grid > 0 && blocks > grid) blocks = grid;
-  k_step_periodic_closure<<<(unsigned)blocks, 32 * width, 0, (cudaStream_t)stream>>>((const S*)f, (S*)fnew,
-                                                                                             a, c);
+  auto* kernel = narrow ? k_step_periodic_closure<true> : k_step_periodic_closure<false>;
+  kernel<<<(unsigned)blocks, 32 * width, 0, (cudaStream_t)stream>>>((const S*)f, (S*)fnew, a, c);
   return lbm::launch_check(who);
 }
 
