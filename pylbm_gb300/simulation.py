@@ -13,9 +13,9 @@ on the device in the padded structure-of-arrays layout of the C ABI; a step is
 
 and a domain that is periodic along every axis skips the first two and uses
 ``lbm_one_time_step_periodic``, which wraps the pull inside the interior.
-``run(n)`` replays a captured CUDA graph of two steps (the buffers are back in
-place after two swaps), so a step costs one graph launch instead of one
-Python call and 2 + nmethods kernel launches.
+``run(n)`` advances several steps per launch where the lattice allows it
+(``_multi_mode``) and replays a captured CUDA graph of sixteen launches or
+steps, an even number, after which the populations are back in place.
 
 ``dtype`` selects the storage type: "float64" (FP64 storage and arithmetic,
 the parity path) or "float32"/"float16"/"bfloat16" (values stored as
@@ -930,7 +930,7 @@ class Simulation:
             return 0
         steps -= steps % multi[0].granule
         done = self._replay(steps, 16 * multi[0].margin, ("multi", mode, bytes(multi[0])), prm,
-                            lambda unit: self._enqueue_multi(mode, multi, prm, unit))
+                            lambda unit: self._enqueue_multi(mode, multi, prm, unit), 32 * multi[0].margin)
         if steps > done:
             self._enqueue_multi(mode, multi, prm, steps - done)
         return steps
@@ -949,19 +949,19 @@ class Simulation:
             self._enqueue_step(self._F, self._Fnew, prm)
             self._enqueue_step(self._Fnew, self._F, prm)
 
-    def _replay(self, steps, unit, kind, prm, enqueue, always=False):
+    def _replay(self, steps, unit, kind, prm, enqueue, repay):
         """Advance up to ``steps`` steps by replays of a graph of ``unit`` steps
         (``enqueue(unit)``, which leaves the populations in F); returns their
         number.  A graph of sixteen launches or more is captured once the steps
         so far repay the capture: between graphs the GPU loses about 1.5 us more
         than between launches of one graph, and a graph of two short steps waits
-        for a whole multiple of 2 us."""
+        for a whole multiple of 2 us.  ``repay``: steps from which on that is so."""
         key = (kind, unit, self._F.ptr, self._Fnew.ptr, tuple(prm))
         if steps < unit:
             return 0
         if key not in self._graphs:
             self._graph_steps += steps
-            if not always and self._graph_steps < 2 * unit:
+            if self._graph_steps < repay:
                 return 0
             if len(self._graphs) >= 4:
                 self._drop_graph()
@@ -970,10 +970,11 @@ class Simulation:
             self._graphs[key] = (graph, self.launches - before)
             self.launches = before
         graph, kernels = self._graphs[key]
-        for _ in range(steps // unit):
+        replays = steps // unit
+        for _ in range(replays):
             runtime.check(self._core.lbm_graph_launch(graph, self._stream))
-        self.launches += steps // unit * kernels
-        return steps // unit * unit
+        self.launches += replays * kernels
+        return replays * unit
 
     def _capture(self, enqueue):
         """The work that ``enqueue`` puts on the stream as an executable graph."""
@@ -1001,8 +1002,10 @@ class Simulation:
         if not done:
             kind = ("single", self._folded(), self.batch_boundary, getattr(self, "closure_kernel", None))
             steps = nsteps // 2 * 2
-            for unit in (16, 2):
-                done += self._replay(steps - done, unit, kind, prm, lambda n: self._enqueue_steps(prm, n), unit == 2)
+            # a first run of few steps is quicker in graphs of two (closure step
+            # at 228^2, 53 steps: 0.84 ms with its capture, 0.99 in sixteens)
+            for unit, repay in ((16, 128), (2, 0)):
+                done += self._replay(steps - done, unit, kind, prm, lambda n: self._enqueue_steps(prm, n), repay)
         for _ in range(done):
             self.t += self.dt
         self.nt += done
