@@ -466,11 +466,13 @@ int lbm_one_time_step_periodic(const void* f, void* fnew, const lbm_lattice* lat
 int lbm_one_time_step_walls(const void* f, void* fnew, const lbm_lattice* lat, const double* prm,
                             const double* table, const int32_t* sym, void* stream);
 
-/* Several steps in one launch, for 2D lattices of shifted (FP32-computed)
- * storage whose stencil reaches one node.  Each block keeps a region of the
- * grid in shared memory, advances it and writes the part that stays valid, so
- * a launch reads and writes the populations once for all its steps; the
- * populations are those of single launches bit for bit.  mode:
+/* Several steps in one launch, for lattices of shifted (FP32-computed)
+ * storage whose stencil reaches one node; the populations are those of single
+ * launches bit for bit, and a launch reads and writes them once for all its
+ * steps.  2D: each block keeps a region of the grid in shared memory, advances
+ * it and writes the part that stays valid.  3D (FP32 storage, the plain
+ * collision, the first two modes): each block walks along the outermost axis
+ * and finishes the second step of a plane behind the first.  mode:
  *   LBM_TILE_PERIODIC  periodic along every axis (lbm_one_time_step_periodic)
  *   LBM_TILE_WALLS     bounce-back box walls (lbm_one_time_step_walls, with
  *                      its table and sym)
